@@ -47,6 +47,49 @@ namespace lab
     unsigned   red_grid(int64_t n);
     unsigned   grid_for(int64_t n);
 
+    // Per-precision views of a level's vectors and operator data.
+    template <class T>
+    struct lv;
+    template <>
+    struct lv<double>
+    {
+        static double* x(level_ws& w) { return w.x; }
+        static double* b(level_ws& w) { return w.b; }
+        static double* r(level_ws& w) { return w.r; }
+        static double* t(level_ws& w) { return w.t; }
+        static const double* invd(const lab_csr_impl* A) { return A->invdiag; }
+    };
+    template <>
+    struct lv<float>
+    {
+        static float* x(level_ws& w) { return w.xf; }
+        static float* b(level_ws& w) { return w.bf; }
+        static float* r(level_ws& w) { return w.rf; }
+        static float* t(level_ws& w) { return w.tf; }
+        static const float* invd(const lab_csr_impl* A) { return A->lp.invd32; }
+    };
+
+    // BF16 value storage on the two finest levels (LAB_PREC_FP32_BF16).
+    static inline bool level_bf16(const lab_amg_options* o, int l)
+    {
+        return o->precision == LAB_PREC_FP32_BF16 && l < 2;
+    }
+
+    // Fused tail (cycle_tail.cu): whether levels l+1 .. L of a V-cycle run as one launch,
+    // with (EDGE) or without (INNER) the restriction out of level l and the prolongation
+    // back, and that launch: from level l's residual wr and iterate cur to its corrected
+    // iterate dst, or from level l+1's right-hand side wr to its correction dst.
+    enum
+    {
+        TAIL_NONE,
+        TAIL_INNER,
+        TAIL_EDGE
+    };
+    int tail_ok(const hierarchy_impl* h, const lab_amg_options* o, int l);
+    template <class T>
+    lab_status tail_launch(hierarchy_impl* h, int l, bool edge, const T* wr, const T* cur, T* dst,
+                           const cyc_ctx& c);
+
     __global__ void k_copy_d(double* __restrict__ y, const double* __restrict__ x, int64_t n,
                              const int* skip);
 }

@@ -18,10 +18,11 @@ namespace lab
         float*  bf  = nullptr;
         float*  rf  = nullptr;
         float*  tf  = nullptr;
-        double* xk  = nullptr; // block cycle vectors: m_l x 8 columns, interleaved per row
+        double* xk  = nullptr; // block cycle vectors: m_l x kcols, interleaved per row
         double* bk  = nullptr;
         double* rk  = nullptr;
         double* tk  = nullptr;
+        int     kcols = 0;
         int32_t* colour = nullptr; // multicolour GS: row order by colour
         int32_t* colour_ptr_h = nullptr; // host copy of colour offsets
         int      ncolours = 0;

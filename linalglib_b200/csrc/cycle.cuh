@@ -32,14 +32,59 @@ namespace lab
     // place; reduced-precision cycles run in correction form x += cycle(0; b - A x).
     lab_status cycle_iterate(hierarchy_impl* h, const cyc_ctx& c, const double* b, double* x);
 
-    // Block V-cycle over many right-hand sides (cycle_blk.cu): whether the options
-    // are covered (V-cycle, Jacobi, FP64, 1x1 or dense coarsest solve; call after
-    // cycle_prepare), the block workspace (outside graph capture), and
-    // z[:, k] = cycle(0; r[:, k]) for ncols column-major columns, 8 per pass.
+    // Scalars and flags per system of a segmented PCG or column of a block one.
+    enum
+    {
+        G_GAMMA = 0,
+        G_PQ    = 1,
+        G_RN    = 2,
+        G_R0    = 3,
+        G_GNEW  = 4,
+        G_N     = 8
+    };
+    enum
+    {
+        GF_DONE   = 0,
+        GF_ITER   = 1,
+        GF_CONV   = 2,
+        GF_STATUS = 3,
+        GF_N      = 4
+    };
+
+    // Block vectors (cycle_blk.cu): ld columns interleaved per row.
+    constexpr int     kBlkMax     = 64;  // columns solved together
+    constexpr int64_t kBlkRedGrid = 592; // CTAs of a pass with a reduction (4 per SM)
+    struct blk_red
+    {
+        double*       partial = nullptr; // kBlkRedGrid x ld
+        unsigned int* counter = nullptr;
+        double*       out     = nullptr; // column c's value at out[c * stride]
+        int           stride  = 0;
+        const int*    skip    = nullptr;
+    };
+    lab_status blk_from_columns(const double* x, int64_t ldx, int64_t n, int ncols, int ld,
+                                double* xb, cudaStream_t s);
+    lab_status blk_to_columns(const double* xb, int64_t n, int ncols, int ld, double* x,
+                              int64_t ldx, cudaStream_t s);
+    lab_status blk_norm(int64_t n, int ld, const double* r, const blk_red& red, cudaStream_t s);
+    lab_status blk_init(double* sc, int* sf, int* gflags, int ld, int max_iter, cudaStream_t s);
+    lab_status blk_update(int64_t n, int ld, double* x, double* r, const double* p, const double* q,
+                          double* sc, int* sf, int* gflags, const blk_red& red, double rtol,
+                          double atol, cudaStream_t s);
+    lab_status blk_pupdate(int64_t n, int ld, double* p, const double* z, double* sc, int* sf,
+                           int* gflags, unsigned int* counter, cudaStream_t s);
+    lab_status blk_spmv_dot(const lab_csr_impl* A, int ld, const double* p, double* q,
+                            const blk_red& red, cudaStream_t s);
+    lab_status blk_residual(const lab_csr_impl* A, int ld, const double* x, const double* b,
+                            double* r, cudaStream_t s);
+    // Block V-cycle: whether the options are covered (V-cycle, Jacobi, FP64, 1x1 or
+    // dense coarsest solve; call after cycle_prepare), the block workspace of at least ld
+    // columns (outside graph capture), and z = cycle(0; r) on ld columns, with (z, r) per
+    // column into dot.out when set.
     bool       cycle_block_supported(const hierarchy_impl* h, const lab_amg_options* o);
-    lab_status cycle_prepare_block(hierarchy_impl* h, cudaStream_t s);
-    lab_status cycle_precond_block(hierarchy_impl* h, const cyc_ctx& c, int ncols, const double* r,
-                                   int64_t ldr, double* z, int64_t ldz);
+    lab_status cycle_prepare_block(hierarchy_impl* h, int ld, cudaStream_t s);
+    lab_status cycle_precond_block(hierarchy_impl* h, const cyc_ctx& c, int ld, const double* r,
+                                   double* z, const blk_red& dot);
 
     // deterministic device reductions into r.out (grid <= kRedBlocks)
     lab_status dot_device(int64_t n, const double* x, const double* y, red_buf r, cudaStream_t s);

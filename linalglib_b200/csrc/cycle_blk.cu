@@ -1,408 +1,618 @@
-// Block V-cycle: the AMG preconditioner applied to up to 8 right-hand sides in
-// one pass over every level operator.  Block vectors hold K columns interleaved
-// per row (entry (i, k) at i*K + k), so one gather fetches the K values of a
-// column index with 16-byte loads and each matrix entry read from HBM serves K
-// products.  Every column sees exactly the arithmetic of the single-vector FP64
-// cycle (same fused passes, same schedule and accumulation order per level), so a
-// block application equals K single applications bit for bit (a level forced onto
-// one thread per row with rows longer than 32 entries is the exception: there the
-// block pass uses W lanes per row).  Covered: V-cycle, Jacobi smoothing (any n1,
-// n2, omega), FP64, 1x1 or dense-inverse coarsest solve; anything else is applied
-// column by column by the caller.
+// Block vectors: up to kBlkMax right-hand sides solved together (multi-RHS PCG with
+// the AMG V-cycle).
+//
+// A block vector holds the ld columns interleaved per row (entry (i, c) at i*ld + c,
+// ld even, columns beyond the caller's zero), in every vector of the solve, so a
+// gather of one matrix entry is one run of 8*ld bytes and each matrix entry read
+// serves all columns.  A thread owns one row and one pair of columns (16-byte loads);
+// the ld/2 threads of a row read the same entry (one broadcast request) and
+// neighbouring pairs of the gathered row.
+//
+// Sums run in CSR order per column (row split into W interleaved parts, added in
+// order, where a level has too few rows to fill the GPU).  Covered: V-cycle, Jacobi
+// smoothing (any n1, n2, omega), FP64, 1x1 or dense-inverse coarsest solve; anything
+// else is applied column by column by the caller.
+//
+// Measured, 32 right-hand sides on a 64^3 Poisson system: groups of 8 columns, one
+// thread per row with 8 accumulators and conversions to and from the block layout
+// around every cycle, 55.6 ms (120 launches and 2 ms an iteration; a warp's 16-byte
+// load of 32 separate rows is 32 lookups); this layout 28.6 ms.
 #include "cycle.cuh"
 
-#include <map>
-#include <mutex>
+#include <algorithm>
 
 namespace lab
 {
-    constexpr int kBlkMax = 8;
+    constexpr int kBlkNT = 256;
 
-    template <int K>
-    __device__ __forceinline__ void ldk(const double* __restrict__ p, double (&o)[K])
+    __device__ __forceinline__ double2 ld2(const double* p)
     {
-        if constexpr(K % 2 == 0)
-        {
-#pragma unroll
-            for(int k = 0; k < K; k += 2)
-            {
-                const double2 t = __ldg(reinterpret_cast<const double2*>(p + k));
-                o[k]            = t.x;
-                o[k + 1]        = t.y;
-            }
-        }
-        else
-        {
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                o[k] = __ldg(p + k);
-        }
+        return __ldg(reinterpret_cast<const double2*>(p));
+    }
+    __device__ __forceinline__ void st2(double* p, double2 v)
+    {
+        *reinterpret_cast<double2*>(p) = v;
+    }
+    __device__ __forceinline__ double2 mul2(double a, double2 v)
+    {
+        return {a * v.x, a * v.y};
     }
 
     // ------------------------------------------------------------ block ops
-    // Same formulas as op_pre0 / op_jacobi / op_res / op_prolong / op_restrict.
-    template <int K>
+    // Same formulas as op_pre0 / op_jacobi / op_res / op_prolong / op_restrict, on one
+    // pair of columns.  at: the pair's offset in row i.
     struct bop_pre0
     {
+        static constexpr bool kDot = false;
         const double* __restrict__ b;
         const double* __restrict__ invd;
         double omega;
         double* __restrict__ x;
         double* __restrict__ r;
-        __device__ __forceinline__ void gather(int c, double (&g)[K]) const
+        struct pre_t
         {
-            double bv[K];
-            ldk<K>(b + (size_t)c * K, bv);
-            const double ic = __ldg(invd + c);
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                g[k] = omega * (ic * bv[k]);
+            double2 b;
+            double  invd;
+        };
+        __device__ __forceinline__ pre_t pre(int i, size_t at) const
+        {
+            return {ld2(b + at), __ldg(invd + i)};
         }
-        __device__ __forceinline__ void finish(int i, const double (&s)[K]) const
+        __device__ __forceinline__ double2 gather(int c, size_t at) const
         {
-            double bv[K];
-            ldk<K>(b + (size_t)i * K, bv);
-            const double ii = __ldg(invd + i);
-#pragma unroll
-            for(int k = 0; k < K; k++)
-            {
-                x[(size_t)i * K + k] = omega * (ii * bv[k]);
-                r[(size_t)i * K + k] = bv[k] - s[k];
-            }
+            return mul2(omega, mul2(__ldg(invd + c), ld2(b + at)));
+        }
+        __device__ __forceinline__ double2 finish(size_t at, double2 s, const pre_t& p) const
+        {
+            st2(x + at, mul2(omega, mul2(p.invd, p.b)));
+            st2(r + at, {p.b.x - s.x, p.b.y - s.y});
+            return {0.0, 0.0};
         }
     };
 
-    template <int K>
+    template <bool DOT>
     struct bop_jacobi
     {
+        static constexpr bool kDot = DOT; // (y, b) per column
         const double* __restrict__ x;
         const double* __restrict__ b;
         const double* __restrict__ invd;
         double omega;
         double* __restrict__ y;
-        __device__ __forceinline__ void gather(int c, double (&g)[K]) const
+        struct pre_t
         {
-            ldk<K>(x + (size_t)c * K, g);
+            double2 x, b;
+            double  invd;
+        };
+        __device__ __forceinline__ pre_t pre(int i, size_t at) const
+        {
+            return {ld2(x + at), ld2(b + at), __ldg(invd + i)};
         }
-        __device__ __forceinline__ void finish(int i, const double (&s)[K]) const
+        __device__ __forceinline__ double2 gather(int, size_t at) const
         {
-            double xv[K], bv[K];
-            ldk<K>(x + (size_t)i * K, xv);
-            ldk<K>(b + (size_t)i * K, bv);
-            const double ii = __ldg(invd + i);
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                y[(size_t)i * K + k] = xv[k] + omega * (ii * (bv[k] - s[k]));
+            return ld2(x + at);
+        }
+        __device__ __forceinline__ double2 finish(size_t at, double2 s, const pre_t& p) const
+        {
+            const double2 v{p.x.x + omega * (p.invd * (p.b.x - s.x)),
+                            p.x.y + omega * (p.invd * (p.b.y - s.y))};
+            st2(y + at, v);
+            return {v.x * p.b.x, v.y * p.b.y};
         }
     };
 
-    template <int K>
     struct bop_res
     {
+        static constexpr bool kDot = false;
         const double* __restrict__ x;
         const double* __restrict__ b;
         double* __restrict__ r;
-        __device__ __forceinline__ void gather(int c, double (&g)[K]) const
+        using pre_t = double2;
+        __device__ __forceinline__ pre_t pre(int, size_t at) const
         {
-            ldk<K>(x + (size_t)c * K, g);
+            return ld2(b + at);
         }
-        __device__ __forceinline__ void finish(int i, const double (&s)[K]) const
+        __device__ __forceinline__ double2 gather(int, size_t at) const
         {
-            double bv[K];
-            ldk<K>(b + (size_t)i * K, bv);
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                r[(size_t)i * K + k] = bv[k] - s[k];
+            return ld2(x + at);
+        }
+        __device__ __forceinline__ double2 finish(size_t at, double2 s, const pre_t& p) const
+        {
+            st2(r + at, {p.x - s.x, p.y - s.y});
+            return {0.0, 0.0};
         }
     };
 
-    // y = x + P e; x and y may alias (each row reads and writes only its own entries)
-    template <int K>
+    // y = x + P e
     struct bop_prolong
     {
+        static constexpr bool kDot = false;
         const double* __restrict__ e;
-        const double* x;
-        double*       y;
-        __device__ __forceinline__ void gather(int c, double (&g)[K]) const
+        const double* __restrict__ x;
+        double* __restrict__ y;
+        using pre_t = double2;
+        __device__ __forceinline__ pre_t pre(int, size_t at) const
         {
-            ldk<K>(e + (size_t)c * K, g);
+            return ld2(x + at);
         }
-        __device__ __forceinline__ void finish(int i, const double (&s)[K]) const
+        __device__ __forceinline__ double2 gather(int, size_t at) const
         {
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                y[(size_t)i * K + k] = x[(size_t)i * K + k] + s[k];
+            return ld2(e + at);
+        }
+        __device__ __forceinline__ double2 finish(size_t at, double2 s, const pre_t& p) const
+        {
+            st2(y + at, {p.x + s.x, p.y + s.y});
+            return {0.0, 0.0};
         }
     };
 
-    template <int K>
+    // y = R r; with x0, also the coarse level's first sweep x0 = omega D_c^-1 y
     struct bop_restrict
     {
+        static constexpr bool kDot = false;
         const double* __restrict__ r;
         double* __restrict__ y;
-        __device__ __forceinline__ void gather(int c, double (&g)[K]) const
+        const double* __restrict__ invd_c;
+        double omega;
+        double* __restrict__ x0;
+        using pre_t = double;
+        __device__ __forceinline__ pre_t pre(int i, size_t) const
         {
-            ldk<K>(r + (size_t)c * K, g);
+            return x0 ? __ldg(invd_c + i) : 0.0;
         }
-        __device__ __forceinline__ void finish(int i, const double (&s)[K]) const
+        __device__ __forceinline__ double2 gather(int, size_t at) const
         {
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                y[(size_t)i * K + k] = s[k];
+            return ld2(r + at);
+        }
+        __device__ __forceinline__ double2 finish(size_t at, double2 s, const pre_t& p) const
+        {
+            st2(y + at, s);
+            if(x0)
+                st2(x0 + at, mul2(omega, mul2(p, s)));
+            return {0.0, 0.0};
         }
     };
 
-    // ------------------------------------------------------------ block row kernels
-    // One thread per row over staged tiles (the ROWSEQ schedule of k_pipe, with K
-    // accumulators): CSR-order fma chains, gathers issued CH entries at a time.
-    template <class Op, int NT, int MAXR, int K>
-    __global__ void __launch_bounds__(NT)
-        k_blk_pipe(csr_view<double> A, Op op, int cap, int ntiles, const int* skip)
+    // q = A p with (p, q) per column
+    struct bop_spmv_dot
     {
-        constexpr int VPC = 2;
-        constexpr int CH  = (16 / K) > 0 ? 16 / K : 1;
-        extern __shared__ __align__(16) unsigned char smem_raw[];
-        const size_t sv_b    = ((size_t)(cap + 16) * sizeof(double) + 15) / 16 * 16;
-        const size_t sc_b    = ((size_t)(cap + 16) * 4 + 15) / 16 * 16;
-        const size_t stage_b = pipe_stage_bytes<double>(cap, NT);
-        if(skip && *skip)
-            return;
-        auto issue = [&](int tile, int stage) {
-            const int      r0   = tile * NT;
-            const int      r1   = min(r0 + NT, A.m);
-            const int      j0   = A.rp[r0];
-            const int      j1   = A.rp[r1];
-            const int      j0v  = j0 & ~(VPC - 1), j0c = j0 & ~3;
-            unsigned char* base = smem_raw + stage * stage_b;
-            int32_t*       sr   = reinterpret_cast<int32_t*>(base + sv_b + sc_b);
-            const int      nr   = (r1 - r0 + 1 + 3) / 4;
-            for(int k = threadIdx.x; k < nr; k += NT)
-                cp_async16(sr + 4 * k, A.rp + r0 + 4 * k);
-            if((j1 - j0v) <= cap + 8 && (j1 - j0c) <= cap + 4)
-            {
-                double*   sv = reinterpret_cast<double*>(base);
-                int32_t*  sc = reinterpret_cast<int32_t*>(base + sv_b);
-                const int nv = (j1 - j0v + VPC - 1) / VPC;
-                const int nc = (j1 - j0c + 3) / 4;
-                for(int k = threadIdx.x; k < nv; k += NT)
-                    cp_async16(sv + (size_t)k * VPC, A.v + j0v + (size_t)k * VPC);
-                for(int k = threadIdx.x; k < nc; k += NT)
-                    cp_async16(sc + (size_t)k * 4, A.ci + j0c + (size_t)k * 4);
-            }
-        };
-        int tile = blockIdx.x;
-        if(tile < ntiles)
-            issue(tile, 0);
-        cp_async_commit();
-        for(int it = 0; tile < ntiles; it++, tile += gridDim.x)
+        static constexpr bool kDot = true;
+        const double* __restrict__ p;
+        double* __restrict__ q;
+        using pre_t = double2;
+        __device__ __forceinline__ pre_t pre(int, size_t at) const
         {
-            const int nxt = tile + gridDim.x;
-            if(nxt < ntiles)
-                issue(nxt, (it + 1) & 1);
-            cp_async_commit();
-            cp_async_wait_group<1>();
-            __syncthreads();
-            const unsigned char* base   = smem_raw + (it & 1) * stage_b;
-            const double*        sv     = reinterpret_cast<const double*>(base);
-            const int32_t*       sc     = reinterpret_cast<const int32_t*>(base + sv_b);
-            const int32_t*       sr     = reinterpret_cast<const int32_t*>(base + sv_b + sc_b);
-            const int            r0     = tile * NT;
-            const int            r1     = min(r0 + NT, A.m);
-            const int            j0     = sr[0], j1 = sr[r1 - r0];
-            const int            j0v    = j0 & ~(VPC - 1), j0c = j0 & ~3;
-            const bool           staged = (j1 - j0v) <= cap + 8 && (j1 - j0c) <= cap + 4;
-            const int            row    = r0 + threadIdx.x;
-            if(row < r1)
+            return ld2(p + at);
+        }
+        __device__ __forceinline__ double2 gather(int, size_t at) const
+        {
+            return ld2(p + at);
+        }
+        __device__ __forceinline__ double2 finish(size_t at, double2 s, const pre_t& pi) const
+        {
+            st2(q + at, s);
+            return {pi.x * s.x, pi.y * s.y};
+        }
+    };
+
+    // ------------------------------------------------------------ reductions
+    __device__ __forceinline__ double2 blk_join(double2 a, double2 b, bool mx)
+    {
+        return mx ? double2{nanmax(a.x, b.x), nanmax(a.y, b.y)} : double2{a.x + b.x, a.y + b.y};
+    }
+
+    // Per-column sum or maximum over the grid: thread t holds the pair t % kl.  The
+    // CTA's partials go to red.partial, the last CTA adds them in order and
+    // calls fin(column, value) once per column from one thread each.
+    template <class F>
+    __device__ __forceinline__ void blk_reduce(double2 acc, int kl, bool mx, const blk_red& red,
+                                               F&& fin)
+    {
+        __shared__ double2 s[kBlkNT];
+        const int          t = threadIdx.x, slots = kBlkNT / kl, ld = 2 * kl;
+        s[t] = acc;
+        __syncthreads();
+        if(t < kl)
+        {
+            double2 v = s[t];
+            for(int q = 1; q < slots; q++)
+                v = blk_join(v, s[q * kl + t], mx);
+            st2(red.partial + (size_t)blockIdx.x * ld + 2 * t, v);
+        }
+        if(!grid_ticket(red.counter))
+            return;
+        double2 v{0.0, 0.0};
+        if(t < slots * kl)
+        {
+            const double* p = red.partial + 2 * (t % kl);
+#pragma unroll 4
+            for(int b = t / kl; b < (int)gridDim.x; b += slots)
+                v = blk_join(v, __ldcg(reinterpret_cast<const double2*>(p + (size_t)b * ld)), mx);
+        }
+        s[t] = v;
+        __syncthreads();
+        if(t < kl)
+        {
+            for(int q = 1; q < slots; q++)
+                v = blk_join(v, s[q * kl + t], mx);
+            fin(2 * t, v.x);
+            fin(2 * t + 1, v.y);
+        }
+        if(t == 0)
+            *red.counter = 0;
+    }
+
+    // ------------------------------------------------------------ row kernel
+    // Threads of a CTA: (row slot, part of the row, column pair), the pair fastest.
+    // The next entries' columns and values are loaded while the gathers of the
+    // current ones are in flight.
+    template <class Op, class IT>
+    __global__ void __launch_bounds__(kBlkNT)
+        k_blk_rows(csr_view<double, IT> A, Op op, int kl, int W, blk_red red)
+    {
+        constexpr int U = 4;
+        if(red.skip && *red.skip)
+            return;
+        __shared__ double2 part[kBlkNT];
+        const int          per  = kBlkNT / (kl * W); // rows of a CTA pass
+        const int          pair = (int)threadIdx.x % kl;
+        const int          w    = ((int)threadIdx.x / kl) % W;
+        const int          slot = (int)threadIdx.x / (kl * W);
+        const size_t       ld   = 2 * (size_t)kl;
+        double2            acc{0.0, 0.0};
+        for(int64_t base = (int64_t)blockIdx.x * per; base < A.m; base += (int64_t)gridDim.x * per)
+        {
+            const bool         valid = slot < per && base + slot < A.m;
+            const int          row   = valid ? (int)(base + slot) : 0;
+            const size_t       at    = (size_t)row * ld + 2 * pair;
+            double2            s{0.0, 0.0};
+            typename Op::pre_t pr{};
+            if(valid)
             {
-                const int a = sr[row - r0], b = sr[row - r0 + 1];
-                double    s[K];
+                const int b = A.rp[row + 1];
+                int       j = A.rp[row] + w;
+                if(w == 0)
+                    pr = op.pre(row, at);
+                double v[U];
+                int    c[U];
 #pragma unroll
-                for(int k = 0; k < K; k++)
-                    s[k] = 0.0;
-                if(staged)
-                {
-                    for(int c0 = a; c0 < b; c0 += CH)
+                for(int u = 0; u < U; u++)
+                    if(j + u * W < b)
                     {
-                        double g[CH][K];
+                        v[u] = __ldg(A.v + j + u * W);
+                        c[u] = col_of<IT>(__ldg(A.ci + j + u * W), row);
+                    }
+#pragma unroll 1
+                for(; j < b; j += U * W)
+                {
+                    double2 g[U];
+                    double  vn[U];
+                    int     cn[U];
 #pragma unroll
-                        for(int q = 0; q < CH; q++)
-                            if(c0 + q < b)
-                                op.gather(sc[c0 + q - j0c], g[q]);
+                    for(int u = 0; u < U; u++)
+                        if(j + u * W < b)
+                            g[u] = op.gather(c[u], (size_t)c[u] * ld + 2 * pair);
 #pragma unroll
-                        for(int q = 0; q < CH; q++)
-                            if(c0 + q < b)
-                            {
-                                const double v = sv[c0 + q - j0v];
+                    for(int u = 0; u < U; u++)
+                        if(j + (U + u) * W < b)
+                        {
+                            vn[u] = __ldg(A.v + j + (U + u) * W);
+                            cn[u] = col_of<IT>(__ldg(A.ci + j + (U + u) * W), row);
+                        }
 #pragma unroll
-                                for(int k = 0; k < K; k++)
-                                    s[k] = fma(v, g[q][k], s[k]);
-                            }
+                    for(int u = 0; u < U; u++)
+                        if(j + u * W < b)
+                        {
+                            s.x = fma(v[u], g[u].x, s.x);
+                            s.y = fma(v[u], g[u].y, s.y);
+                        }
+#pragma unroll
+                    for(int u = 0; u < U; u++)
+                    {
+                        v[u] = vn[u];
+                        c[u] = cn[u];
                     }
                 }
-                else
-                {
-                    for(int j = a; j < b; j++)
-                    {
-                        double g[K];
-                        op.gather(A.ci[j], g);
-                        const double v = A.v[j];
-#pragma unroll
-                        for(int k = 0; k < K; k++)
-                            s[k] = fma(v, g[k], s[k]);
-                    }
-                }
-                op.finish(row, s);
             }
-            __syncthreads();
-        }
-        cp_async_wait_group<0>();
-    }
-
-    // W lanes per row, lane-strided partial sums and an xor-shuffle reduction per
-    // column (the VECTOR schedule of k_vector with K accumulators).
-    template <class Op, int NT, int W, int K>
-    __global__ void __launch_bounds__(NT)
-        k_blk_vector(csr_view<double> A, Op op, const int* skip)
-    {
-        if(skip && *skip)
-            return;
-        const int lane = threadIdx.x & (W - 1);
-        const int row  = (int)(((int64_t)blockIdx.x * NT + threadIdx.x) / W);
-        double    s[K];
-#pragma unroll
-        for(int k = 0; k < K; k++)
-            s[k] = 0.0;
-        if(row < A.m)
-        {
-            const int a = A.rp[row], b = A.rp[row + 1];
-            for(int j = a + lane; j < b; j += W)
+            if(W > 1)
             {
-                double g[K];
-                op.gather(A.ci[j], g);
-                const double v = A.v[j];
-#pragma unroll
-                for(int k = 0; k < K; k++)
-                    s[k] = fma(v, g[k], s[k]);
+                part[threadIdx.x] = s;
+                __syncthreads();
+                if(valid && w == 0)
+                    for(int q = 1; q < W; q++)
+                        s = blk_join(s, part[threadIdx.x + q * kl], false);
+                __syncthreads();
+            }
+            if(valid && w == 0)
+            {
+                const double2 d = op.finish(at, s, pr);
+                if(Op::kDot)
+                {
+                    acc.x += d.x;
+                    acc.y += d.y;
+                }
             }
         }
-#pragma unroll
-        for(int k = 0; k < K; k++)
-#pragma unroll
-            for(int o = W / 2; o > 0; o >>= 1)
-                s[k] += __shfl_xor_sync(0xffffffffu, s[k], o, W);
-        if(row < A.m && lane == 0)
-            op.finish(row, s);
+        if(Op::kDot)
+            blk_reduce(acc, kl, false, red,
+                       [&](int c, double v) { red.out[(size_t)c * red.stride] = v; });
     }
 
-    template <class Op, int MAXR, int K>
-    static int blk_pipe_occupancy(size_t smem)
-    {
-        const auto                   kernel = k_blk_pipe<Op, kRowseqNT, MAXR, K>;
-        static std::mutex            mu;
-        static std::map<size_t, int> cache;
-        static const cudaError_t     attr = cudaFuncSetAttribute(
-            kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        (void)attr;
-        std::lock_guard<std::mutex> g(mu);
-        auto                        it = cache.find(smem);
-        if(it != cache.end())
-            return it->second;
-        int occ = 0;
-        if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, kRowseqNT, smem) !=
-           cudaSuccess)
-        {
-            cudaGetLastError();
-            occ = 1;
-        }
-        occ         = std::max(occ, 1);
-        cache[smem] = occ;
-        return occ;
-    }
-
-    template <class Op, int MAXR, int K>
-    static lab_status blk_pipe(const csr_view<double>& V, const Op& op, int cap, cudaStream_t s,
-                               const int* skip)
-    {
-        const int      ntiles = (int)ceil_div<int64_t>(V.m, kRowseqNT);
-        const size_t   smem   = 2 * pipe_stage_bytes<double>(cap, kRowseqNT);
-        const int      occ    = blk_pipe_occupancy<Op, MAXR, K>(smem);
-        const unsigned grid   = (unsigned)std::min<int64_t>(ntiles, (int64_t)num_sms() * occ);
-        LAB_LAUNCH((k_blk_pipe<Op, kRowseqNT, MAXR, K>), grid, kRowseqNT, smem, s, V, op, cap,
-                   ntiles, skip);
-        return LAB_OK;
-    }
-
-    template <class Op, int W, int K>
-    static lab_status blk_vector(const csr_view<double>& V, const Op& op, cudaStream_t s,
-                                 const int* skip)
-    {
-        const unsigned grid = (unsigned)ceil_div<int64_t>((int64_t)V.m * W, kVectorNT);
-        LAB_LAUNCH((k_blk_vector<Op, kVectorNT, W, K>), grid, kVectorNT, 0, s, V, op, skip);
-        return LAB_OK;
-    }
-
-    // The schedule of the matrix's SpMV plan, with K accumulators.
-    template <int K, class Op>
-    static lab_status blk_rowop(const lab_csr_impl* A, const Op& op, cudaStream_t s,
-                                const int* skip)
+    // W: interleaved parts of a row.  Below about 1024 threads per SM the pass waits on
+    // the row -> entries -> gathers chain, so rows are split until the grid reaches
+    // that or a part is down to four entries.
+    template <class Op>
+    static lab_status blk_rows(const lab_csr_impl* A, const Op& op, int ld, cudaStream_t s,
+                               const blk_red& red)
     {
         if(A->m == 0)
             return LAB_OK;
-        csr_view<double> V{A->row_ptr, A->col_ind, A->val, (int32_t)A->m};
-        const spmv_plan& p = A->plan;
-        if(p.alg == LAB_SPMV_ROWSEQ)
+        const int kl = ld / 2;
+        int       W  = 1;
+        while(W < 16 && 2 * W * kl <= kBlkNT && A->m * kl * W < (int64_t)num_sms() * 1024 &&
+              A->nnz >= 8 * A->m * W)
+            W *= 2;
+        const int64_t  per  = kBlkNT / (kl * W);
+        const unsigned grid = (unsigned)std::min<int64_t>(
+            ceil_div<int64_t>(A->m, per), Op::kDot ? kBlkRedGrid : (int64_t)num_sms() * 32);
+        if(A->lp.dcol)
         {
-            const int mr = std::max(1, p.max_row);
-            if(mr <= 8)
-                return blk_pipe<Op, 8, K>(V, op, kRowseqNT * mr, s, skip);
-            if(mr <= 16)
-                return blk_pipe<Op, 16, K>(V, op, kRowseqNT * mr, s, skip);
-            if(mr <= 32)
-                return blk_pipe<Op, 32, K>(V, op, kRowseqNT * mr, s, skip);
+            csr_view<double, int16_t> V{A->row_ptr, A->lp.dcol, A->val, (int32_t)A->m};
+            LAB_LAUNCH((k_blk_rows<Op, int16_t>), grid, kBlkNT, 0, s, V, op, kl, W, red);
         }
-        // long rows: W lanes per row, as the single-vector VECTOR schedule
-        switch(p.alg == LAB_SPMV_VECTOR ? p.lanes : p.vlanes)
+        else
         {
-        case 2:
-            return blk_vector<Op, 2, K>(V, op, s, skip);
-        case 4:
-            return blk_vector<Op, 4, K>(V, op, s, skip);
-        case 8:
-            return blk_vector<Op, 8, K>(V, op, s, skip);
-        case 16:
-            return blk_vector<Op, 16, K>(V, op, s, skip);
-        default:
-            return blk_vector<Op, 32, K>(V, op, s, skip);
+            csr_view<double, int32_t> V{A->row_ptr, A->col_ind, A->val, (int32_t)A->m};
+            LAB_LAUNCH((k_blk_rows<Op, int32_t>), grid, kBlkNT, 0, s, V, op, kl, W, red);
         }
+        return LAB_OK;
+    }
+
+    // ------------------------------------------------------------ layout
+    // Column-major columns to interleaved and back, 32 rows by up to 32 columns through
+    // shared memory so both sides are coalesced.
+    __global__ void k_to_blk(const double* __restrict__ x, int64_t ldx, int64_t n, int ncols,
+                             int ld, double* __restrict__ xb)
+    {
+        __shared__ double t[32][33];
+        const int64_t     i0 = (int64_t)blockIdx.x * 32;
+        for(int c0 = 0; c0 < ld; c0 += 32)
+        {
+            for(int c = c0 + threadIdx.y; c < min(c0 + 32, ld); c += blockDim.y)
+                t[c - c0][threadIdx.x] =
+                    c < ncols && i0 + threadIdx.x < n ? x[c * ldx + i0 + threadIdx.x] : 0.0;
+            __syncthreads();
+            for(int r = threadIdx.y; r < 32; r += blockDim.y)
+                if(i0 + r < n && c0 + (int)threadIdx.x < ld)
+                    xb[(i0 + r) * ld + c0 + threadIdx.x] = t[threadIdx.x][r];
+            __syncthreads();
+        }
+    }
+
+    __global__ void k_from_blk(const double* __restrict__ xb, int64_t n, int ncols, int ld,
+                               double* __restrict__ x, int64_t ldx)
+    {
+        __shared__ double t[32][33];
+        const int64_t     i0 = (int64_t)blockIdx.x * 32;
+        for(int c0 = 0; c0 < ncols; c0 += 32)
+        {
+            for(int r = threadIdx.y; r < 32; r += blockDim.y)
+                if(i0 + r < n && c0 + (int)threadIdx.x < ncols)
+                    t[r][threadIdx.x] = xb[(i0 + r) * ld + c0 + threadIdx.x];
+            __syncthreads();
+            for(int c = c0 + threadIdx.y; c < min(c0 + 32, ncols); c += blockDim.y)
+                if(i0 + threadIdx.x < n)
+                    x[c * ldx + i0 + threadIdx.x] = t[threadIdx.x][c - c0];
+            __syncthreads();
+        }
+    }
+
+    lab_status blk_from_columns(const double* x, int64_t ldx, int64_t n, int ncols, int ld,
+                                double* xb, cudaStream_t s)
+    {
+        LAB_LAUNCH(k_to_blk, (unsigned)ceil_div<int64_t>(n, 32), dim3(32, 8), 0, s, x, ldx, n, ncols,
+                   ld, xb);
+        return LAB_OK;
+    }
+
+    lab_status blk_to_columns(const double* xb, int64_t n, int ncols, int ld, double* x,
+                              int64_t ldx, cudaStream_t s)
+    {
+        LAB_LAUNCH(k_from_blk, (unsigned)ceil_div<int64_t>(n, 32), dim3(32, 8), 0, s, xb, n, ncols,
+                   ld, x, ldx);
+        return LAB_OK;
+    }
+
+    // ------------------------------------------------------------ PCG vector passes
+    __device__ __forceinline__ void blk_retire(int* sf, int c, int* gflags, int status, int conv)
+    {
+        sf[c * GF_N + GF_DONE]   = 1;
+        sf[c * GF_N + GF_CONV]   = conv;
+        sf[c * GF_N + GF_STATUS] = status;
+        if(atomicSub(&gflags[1], 1) == 1)
+            gflags[0] = 1;
+    }
+
+    // ||r||_inf per column into sc[c][G_R0]
+    __global__ void __launch_bounds__(kBlkNT)
+        k_blk_norm(int64_t n, int kl, const double* __restrict__ r, blk_red red)
+    {
+        const int    pair = (int)threadIdx.x % kl, slot = (int)threadIdx.x / kl;
+        const int    per  = kBlkNT / kl;
+        double2      acc{0.0, 0.0};
+        if(slot < per)
+            for(int64_t i = (int64_t)blockIdx.x * per + slot; i < n; i += (int64_t)gridDim.x * per)
+            {
+                const double2 v = ld2(r + i * 2 * kl + 2 * pair);
+                acc             = blk_join(acc, {fabs(v.x), fabs(v.y)}, true);
+            }
+        blk_reduce(acc, kl, true, red,
+                   [&](int c, double v) { red.out[(size_t)c * red.stride] = v; });
+    }
+
+    // gamma = (z, r), p = z is set by the caller; columns with r = 0 retire at once.
+    __global__ void k_blk_init(double* sc, int* sf, int* gflags, int ld, int max_iter)
+    {
+        int active = 0;
+        for(int c = threadIdx.x; c < ld; c += 32)
+        {
+            sc[c * G_N + G_GAMMA]    = sc[c * G_N + G_GNEW];
+            sc[c * G_N + G_RN]       = sc[c * G_N + G_R0];
+            const bool zero          = sc[c * G_N + G_R0] == 0.0;
+            sf[c * GF_N + GF_ITER]   = 0;
+            sf[c * GF_N + GF_DONE]   = zero;
+            sf[c * GF_N + GF_CONV]   = zero;
+            sf[c * GF_N + GF_STATUS] = zero ? LAB_OK : LAB_NOT_CONVERGED;
+            active += !zero;
+        }
+        for(int o = 16; o > 0; o >>= 1)
+            active += __shfl_xor_sync(0xffffffffu, active, o);
+        if(threadIdx.x == 0)
+        {
+            gflags[1] = active;
+            gflags[2] = max_iter;
+            gflags[0] = active == 0;
+        }
+    }
+
+    // x += alpha p; r -= alpha q; ||r||_inf; stopping test, per column (k_seg_update)
+    __global__ void __launch_bounds__(kBlkNT)
+        k_blk_update(int64_t n, int kl, double* __restrict__ x, double* __restrict__ r,
+                     const double* __restrict__ p, const double* __restrict__ q, double* sc, int* sf,
+                     int* gflags, blk_red red, double rtol, double atol)
+    {
+        if(gflags[0])
+            return;
+        const int    pair = (int)threadIdx.x % kl, slot = (int)threadIdx.x / kl;
+        const int    per  = kBlkNT / kl;
+        const int    c0   = 2 * pair;
+        const bool   d0 = sf[c0 * GF_N + GF_DONE], d1 = sf[(c0 + 1) * GF_N + GF_DONE];
+        const double a0 = sc[c0 * G_N + G_GAMMA] / sc[c0 * G_N + G_PQ];
+        const double a1 = sc[(c0 + 1) * G_N + G_GAMMA] / sc[(c0 + 1) * G_N + G_PQ];
+        double2      acc{0.0, 0.0};
+        if(slot < per && !(d0 && d1))
+        {
+#pragma unroll 2
+            for(int64_t i = (int64_t)blockIdx.x * per + slot; i < n; i += (int64_t)gridDim.x * per)
+            {
+                const size_t  at = (size_t)i * 2 * kl + c0;
+                const double2 pv = ld2(p + at), qv = ld2(q + at);
+                double2       xv = *reinterpret_cast<const double2*>(x + at);
+                double2       rv = *reinterpret_cast<const double2*>(r + at);
+                if(!d0)
+                {
+                    xv.x = __dadd_rn(__dmul_rn(a0, pv.x), xv.x);
+                    rv.x = __dadd_rn(__dmul_rn(-a0, qv.x), rv.x);
+                }
+                if(!d1)
+                {
+                    xv.y = __dadd_rn(__dmul_rn(a1, pv.y), xv.y);
+                    rv.y = __dadd_rn(__dmul_rn(-a1, qv.y), rv.y);
+                }
+                st2(x + at, xv);
+                st2(r + at, rv);
+                acc = blk_join(acc, {fabs(rv.x), fabs(rv.y)}, true);
+            }
+        }
+        blk_reduce(acc, kl, true, red, [&](int c, double t) {
+            if(sf[c * GF_N + GF_DONE])
+                return;
+            sc[c * G_N + G_RN] = t;
+            const double r0    = sc[c * G_N + G_R0];
+            const bool   nan   = isnan(t) || isnan(r0);
+            if(!nan && (t <= atol || t / r0 <= rtol))
+                blk_retire(sf, c, gflags, LAB_OK, 1);
+            else if(nan)
+                blk_retire(sf, c, gflags, LAB_NAN, 0);
+        });
+    }
+
+    // p = z + beta p, then (last CTA) gamma <- gnew, iteration count, max_iter test
+    __global__ void __launch_bounds__(kBlkNT)
+        k_blk_pupdate(int64_t n, int kl, double* __restrict__ p, const double* __restrict__ z,
+                      double* sc, int* sf, int* gflags, unsigned int* counter)
+    {
+        if(gflags[0])
+            return;
+        const int    pair = (int)threadIdx.x % kl, slot = (int)threadIdx.x / kl;
+        const int    per  = kBlkNT / kl;
+        const int    c0   = 2 * pair;
+        const bool   d0 = sf[c0 * GF_N + GF_DONE], d1 = sf[(c0 + 1) * GF_N + GF_DONE];
+        const double b0 = sc[c0 * G_N + G_GNEW] / sc[c0 * G_N + G_GAMMA];
+        const double b1 = sc[(c0 + 1) * G_N + G_GNEW] / sc[(c0 + 1) * G_N + G_GAMMA];
+        if(slot < per && !(d0 && d1))
+        {
+#pragma unroll 4
+            for(int64_t i = (int64_t)blockIdx.x * per + slot; i < n; i += (int64_t)gridDim.x * per)
+            {
+                const size_t  at = (size_t)i * 2 * kl + c0;
+                const double2 zv = ld2(z + at);
+                double2       pv = *reinterpret_cast<const double2*>(p + at);
+                if(!d0)
+                    pv.x = b0 == 0.0 ? zv.x : __dadd_rn(zv.x, __dmul_rn(b0, pv.x));
+                if(!d1)
+                    pv.y = b1 == 0.0 ? zv.y : __dadd_rn(zv.y, __dmul_rn(b1, pv.y));
+                st2(p + at, pv);
+            }
+        }
+        if(!grid_ticket(counter))
+            return;
+        for(int c = threadIdx.x; c < 2 * kl; c += kBlkNT)
+            if(!sf[c * GF_N + GF_DONE])
+            {
+                sc[c * G_N + G_GAMMA]  = sc[c * G_N + G_GNEW];
+                const int it           = sf[c * GF_N + GF_ITER] + 1;
+                sf[c * GF_N + GF_ITER] = it;
+                if(it > gflags[2])
+                    blk_retire(sf, c, gflags, LAB_NOT_CONVERGED, 0);
+            }
+        if(threadIdx.x == 0)
+            *counter = 0;
+    }
+
+    static unsigned blk_grid(int64_t n, int kl)
+    {
+        return (unsigned)std::max<int64_t>(
+            1, std::min<int64_t>(ceil_div<int64_t>(n, kBlkNT / kl), kBlkRedGrid));
+    }
+
+    lab_status blk_norm(int64_t n, int ld, const double* r, const blk_red& red, cudaStream_t s)
+    {
+        LAB_LAUNCH(k_blk_norm, blk_grid(n, ld / 2), kBlkNT, 0, s, n, ld / 2, r, red);
+        return LAB_OK;
+    }
+    lab_status blk_init(double* sc, int* sf, int* gflags, int ld, int max_iter, cudaStream_t s)
+    {
+        LAB_LAUNCH(k_blk_init, 1, 32, 0, s, sc, sf, gflags, ld, max_iter);
+        return LAB_OK;
+    }
+    lab_status blk_update(int64_t n, int ld, double* x, double* r, const double* p, const double* q,
+                          double* sc, int* sf, int* gflags, const blk_red& red, double rtol,
+                          double atol, cudaStream_t s)
+    {
+        LAB_LAUNCH(k_blk_update, blk_grid(n, ld / 2), kBlkNT, 0, s, n, ld / 2, x, r, p, q, sc, sf,
+                   gflags, red, rtol, atol);
+        return LAB_OK;
+    }
+    lab_status blk_pupdate(int64_t n, int ld, double* p, const double* z, double* sc, int* sf,
+                           int* gflags, unsigned int* counter, cudaStream_t s)
+    {
+        LAB_LAUNCH(k_blk_pupdate, blk_grid(n, ld / 2), kBlkNT, 0, s, n, ld / 2, p, z, sc, sf,
+                   gflags, counter);
+        return LAB_OK;
+    }
+    lab_status blk_spmv_dot(const lab_csr_impl* A, int ld, const double* p, double* q,
+                            const blk_red& red, cudaStream_t s)
+    {
+        return blk_rows(A, bop_spmv_dot{p, q}, ld, s, red);
+    }
+    lab_status blk_residual(const lab_csr_impl* A, int ld, const double* x, const double* b,
+                            double* r, cudaStream_t s)
+    {
+        return blk_rows(A, bop_res{x, b, r}, ld, s, blk_red{});
     }
 
     // ------------------------------------------------------------ small kernels
-    template <int K>
-    __global__ void k_to_blk(const double* __restrict__ r, int64_t ld, int64_t n,
-                             double* __restrict__ rb, const int* skip)
-    {
-        if(skip && *skip)
-            return;
-        for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-            i += (int64_t)gridDim.x * blockDim.x)
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                rb[i * K + k] = r[k * ld + i];
-    }
-
-    template <int K>
-    __global__ void k_from_blk(const double* __restrict__ zb, int64_t n, double* __restrict__ z,
-                               int64_t ld, const int* skip)
-    {
-        if(skip && *skip)
-            return;
-        for(int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-            i += (int64_t)gridDim.x * blockDim.x)
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                z[k * ld + i] = zb[i * K + k];
-    }
-
     __global__ void k_blk_zero(double* x, int64_t n, const int* skip)
     {
         if(skip && *skip)
@@ -412,187 +622,166 @@ namespace lab
             x[i] = 0.0;
     }
 
-    template <int K>
-    __global__ void k_blk_coarse1(const double* a, const double* b, double* x, const int* skip)
+    // Coarsest level per column: x = b / a (1x1) or x = Ainv b.
+    __global__ void k_blk_coarse(const double* __restrict__ a, const double* __restrict__ b,
+                                 double* __restrict__ x, int n, int ld, const int* skip)
     {
         if(skip && *skip)
             return;
-        if(threadIdx.x < K)
-            x[threadIdx.x] = __ddiv_rn(b[threadIdx.x], a[0]);
-    }
-
-    // x = Ainv b per column, the single-vector kernel's order (lane-strided fma, warp sum)
-    template <int K>
-    __global__ void k_blk_coarse_dense(const double* __restrict__ Ainv, const double* __restrict__ b,
-                                       double* __restrict__ x, int n, const int* skip)
-    {
-        if(skip && *skip)
-            return;
-        const int row  = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-        const int lane = threadIdx.x & 31;
+        const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+        const int     row = (int)(t / ld), c = (int)(t % ld);
         if(row >= n)
             return;
-        double s[K];
-#pragma unroll
-        for(int k = 0; k < K; k++)
-            s[k] = 0.0;
-        for(int j = lane; j < n; j += 32)
+        if(n == 1)
         {
-            const double a = Ainv[(size_t)row * n + j];
-#pragma unroll
-            for(int k = 0; k < K; k++)
-                s[k] = fma(a, b[(size_t)j * K + k], s[k]);
+            x[c] = __ddiv_rn(b[c], a[0]);
+            return;
         }
-#pragma unroll
-        for(int k = 0; k < K; k++)
-        {
-            const double t = warp_sum(s[k]);
-            if(lane == 0)
-                x[(size_t)row * K + k] = t;
-        }
+        double s = 0.0;
+#pragma unroll 4
+        for(int j = 0; j < n; j++)
+            s = fma(__ldg(a + (size_t)row * n + j), __ldg(b + (size_t)j * ld + c), s);
+        x[(size_t)row * ld + c] = s;
+    }
+
+    // (z, r) where the cycle's last pass does not form it
+    __global__ void __launch_bounds__(kBlkNT)
+        k_blk_dot(int64_t n, int kl, const double* __restrict__ x, const double* __restrict__ y,
+                  blk_red red)
+    {
+        if(red.skip && *red.skip)
+            return;
+        const int    pair = (int)threadIdx.x % kl, slot = (int)threadIdx.x / kl;
+        const int    per  = kBlkNT / kl;
+        double2      acc{0.0, 0.0};
+        if(slot < per)
+            for(int64_t i = (int64_t)blockIdx.x * per + slot; i < n; i += (int64_t)gridDim.x * per)
+            {
+                const double2 u = ld2(x + i * 2 * kl + 2 * pair), v = ld2(y + i * 2 * kl + 2 * pair);
+                acc.x += u.x * v.x;
+                acc.y += u.y * v.y;
+            }
+        blk_reduce(acc, kl, false, red,
+                   [&](int c, double v) { red.out[(size_t)c * red.stride] = v; });
     }
 
     // ------------------------------------------------------------ the recursion
-    template <int K>
-    static lab_status cycle_blk(hierarchy_impl* h, int l, double* x, const double* b,
-                                const cyc_ctx& c)
+    // x = cycle(0; b) on level l; x0_ready: the restriction wrote the first sweep into
+    // the buffer that the cycle starts in; dot (level 0): (x, b) per column.
+    static bool blk_starts_in_t(const lab_amg_options* o)
+    {
+        // start in the buffer that makes the last write land in x
+        return (((o->n1 >= 1 ? o->n1 - 1 : o->n1) + 1 + o->n2) & 1) != 0;
+    }
+
+    static lab_status cycle_blk(hierarchy_impl* h, int l, int ld, double* x, const double* b,
+                                const cyc_ctx& c, bool x0_ready, const blk_red& dot)
     {
         const lab_amg_options* o = c.o;
+        lab_csr_impl*          A = h->A[l];
+        const int64_t          m = A->m;
+        blk_red                none{};
+        none.skip = c.skip;
+        auto dotted = [&]() -> lab_status {
+            if(dot.out)
+                LAB_LAUNCH(k_blk_dot, blk_grid(m, ld / 2), kBlkNT, 0, c.s, m, ld / 2,
+                           (const double*)x, b, dot);
+            return LAB_OK;
+        };
         if(l == h->levels)
         {
-            const lab_csr_impl* A = h->A[l];
-            if(A->m == 1)
-                LAB_LAUNCH(k_blk_coarse1<K>, 1, 32, 0, c.s, (const double*)A->val, b, x, c.skip);
-            else if(A->m > 1)
-                LAB_LAUNCH(k_blk_coarse_dense<K>, (unsigned)ceil_div<int64_t>(A->m, 8), 256, 0, c.s,
-                           (const double*)h->coarse_inv, b, x, (int)A->m, c.skip);
-            return LAB_OK;
+            if(m > 0)
+                LAB_LAUNCH(k_blk_coarse, (unsigned)ceil_div<int64_t>(m * ld, 128), 128, 0, c.s,
+                           (const double*)(m == 1 ? A->val : h->coarse_inv), b, x, (int)m, ld,
+                           c.skip);
+            return dotted();
         }
-        lab_csr_impl* A    = h->A[l];
         lab_csr_impl* P    = h->P[l];
         lab_csr_impl* R    = h->R[l];
         level_ws&     w    = h->ws[l];
         level_ws&     wc   = h->ws[l + 1];
-        const int64_t m    = A->m;
         const int     n1   = o->n1, n2 = o->n2;
         const double  om   = o->omega;
         const double* invd = A->invdiag;
         double*       r    = w.rk;
-        // start in the buffer that makes the last write land in x
-        double*   cur   = x;
-        double*   oth   = w.tk;
-        const int flips = (n1 >= 1 ? n1 - 1 : n1) + 1 + n2;
-        if(flips & 1)
-        {
-            cur = w.tk;
-            oth = x;
-        }
-        auto jacobi = [&]() -> lab_status {
-            bop_jacobi<K> op{cur, b, invd, om, oth};
-            LAB_TRY(blk_rowop<K>(A, op, c.s, c.skip));
+        double*       cur  = x;
+        double*       oth  = w.tk;
+        if(blk_starts_in_t(o))
+            std::swap(cur, oth);
+        auto jacobi = [&](bool last) -> lab_status {
+            if(last && dot.out)
+                LAB_TRY(blk_rows(A, bop_jacobi<true>{cur, b, invd, om, oth}, ld, c.s, dot));
+            else
+                LAB_TRY(blk_rows(A, bop_jacobi<false>{cur, b, invd, om, oth}, ld, c.s, none));
             std::swap(cur, oth);
             return LAB_OK;
         };
         if(n1 >= 1)
         {
-            bop_pre0<K> op{b, invd, om, cur, r};
-            LAB_TRY(blk_rowop<K>(A, op, c.s, c.skip));
+            if(x0_ready)
+                LAB_TRY(blk_rows(A, bop_res{cur, b, r}, ld, c.s, none));
+            else
+                LAB_TRY(blk_rows(A, bop_pre0{b, invd, om, cur, r}, ld, c.s, none));
             for(int k = 1; k < n1; k++)
-                LAB_TRY(jacobi());
+                LAB_TRY(jacobi(false));
             if(n1 > 1)
-            {
-                bop_res<K> opr{cur, b, r};
-                LAB_TRY(blk_rowop<K>(A, opr, c.s, c.skip));
-            }
+                LAB_TRY(blk_rows(A, bop_res{cur, b, r}, ld, c.s, none));
         }
         else
         {
-            LAB_LAUNCH(k_blk_zero, grid_for(m * K), 256, 0, c.s, cur, m * K, c.skip);
-            bop_res<K> opr{cur, b, r};
-            LAB_TRY(blk_rowop<K>(A, opr, c.s, c.skip));
+            LAB_LAUNCH(k_blk_zero, grid_for(m * ld), 256, 0, c.s, cur, m * ld, c.skip);
+            LAB_TRY(blk_rows(A, bop_res{cur, b, r}, ld, c.s, none));
         }
-        bop_restrict<K> opr{r, wc.bk};
-        LAB_TRY(blk_rowop<K>(R, opr, c.s, c.skip));
-        LAB_TRY(cycle_blk<K>(h, l + 1, wc.xk, wc.bk, c));
-        bop_prolong<K> opp{wc.xk, cur, oth};
-        LAB_TRY(blk_rowop<K>(P, opp, c.s, c.skip));
+        const bool fuse = n1 >= 1 && l + 1 < h->levels;
+        double*    x0   = fuse ? (blk_starts_in_t(o) ? wc.tk : wc.xk) : nullptr;
+        LAB_TRY(blk_rows(R, bop_restrict{r, wc.bk, h->A[l + 1]->invdiag, om, x0}, ld, c.s, none));
+        LAB_TRY(cycle_blk(h, l + 1, ld, wc.xk, wc.bk, c, fuse, blk_red{}));
+        LAB_TRY(blk_rows(P, bop_prolong{wc.xk, cur, oth}, ld, c.s, none));
         std::swap(cur, oth);
         for(int k = 0; k < n2; k++)
-            LAB_TRY(jacobi());
+            LAB_TRY(jacobi(k == n2 - 1));
         if(cur != x)
         {
             set_error("block cycle: internal buffer parity");
             return LAB_BAD_ARG;
         }
-        return LAB_OK;
+        return n2 > 0 ? LAB_OK : dotted();
     }
 
     bool cycle_block_supported(const hierarchy_impl* h, const lab_amg_options* o)
     {
         if(o->cycle != LAB_CYCLE_V || o->smoother != LAB_SMOOTH_JACOBI ||
-           o->precision != LAB_PREC_FP64 || o->n1 < 0 || o->n2 < 0)
+           o->precision != LAB_PREC_FP64 || o->n1 < 0 || o->n2 < 0 || h->A[0]->m == 0)
             return false;
         const lab_csr_impl* Ac = h->A[h->levels];
         return Ac->m <= 1 || (o->coarse == LAB_COARSE_DIRECT && h->coarse_inv);
     }
 
-    lab_status cycle_prepare_block(hierarchy_impl* h, cudaStream_t s)
+    lab_status cycle_prepare_block(hierarchy_impl* h, int ld, cudaStream_t s)
     {
         for(int l = 0; l <= h->levels; l++)
         {
-            level_ws&    w = h->ws[l];
-            const size_t n = (size_t)h->A[l]->m * kBlkMax + 8;
-            if(!w.xk)
+            level_ws& w = h->ws[l];
+            if(w.kcols >= ld)
+                continue;
+            double** v[4] = {&w.xk, &w.bk, &w.rk, &w.tk};
+            w.kcols       = 0;
+            for(double** p : v)
             {
-                LAB_TRY(dalloc(&w.xk, n, s));
-                LAB_TRY(dalloc(&w.bk, n, s));
-                LAB_TRY(dalloc(&w.rk, n, s));
-                LAB_TRY(dalloc(&w.tk, n, s));
+                dfree(*p, s);
+                *p = nullptr;
+                // level 0 works on the solve's own vectors and needs scratch alone
+                if(l > 0 || p == &w.rk || p == &w.tk)
+                    LAB_TRY(dalloc(p, (size_t)h->A[l]->m * ld + 2, s));
             }
+            w.kcols = ld;
         }
         return LAB_OK;
     }
 
-    template <int K>
-    static lab_status precond_group(hierarchy_impl* h, const cyc_ctx& c, const double* r,
-                                    int64_t ldr, double* z, int64_t ldz)
+    lab_status cycle_precond_block(hierarchy_impl* h, const cyc_ctx& c, int ld, const double* r,
+                                   double* z, const blk_red& dot)
     {
-        const int64_t n  = h->A[0]->m;
-        level_ws&     w0 = h->ws[0];
-        const unsigned g = grid_for(n);
-        LAB_LAUNCH(k_to_blk<K>, g, 256, 0, c.s, r, ldr, n, w0.bk, c.skip);
-        LAB_TRY(cycle_blk<K>(h, 0, w0.xk, w0.bk, c));
-        LAB_LAUNCH(k_from_blk<K>, g, 256, 0, c.s, (const double*)w0.xk, n, z, ldz, c.skip);
-        return LAB_OK;
-    }
-
-    lab_status cycle_precond_block(hierarchy_impl* h, const cyc_ctx& c, int ncols, const double* r,
-                                   int64_t ldr, double* z, int64_t ldz)
-    {
-        int col = 0;
-        while(col < ncols)
-        {
-            const int left = ncols - col;
-            const int k    = left >= 8 ? 8 : left >= 4 ? 4 : left >= 2 ? 2 : 1;
-            const double* rc = r + (int64_t)col * ldr;
-            double*       zc = z + (int64_t)col * ldz;
-            switch(k)
-            {
-            case 8:
-                LAB_TRY(precond_group<8>(h, c, rc, ldr, zc, ldz));
-                break;
-            case 4:
-                LAB_TRY(precond_group<4>(h, c, rc, ldr, zc, ldz));
-                break;
-            case 2:
-                LAB_TRY(precond_group<2>(h, c, rc, ldr, zc, ldz));
-                break;
-            default:
-                LAB_TRY(precond_group<1>(h, c, rc, ldr, zc, ldz));
-                break;
-            }
-            col += k;
-        }
-        return LAB_OK;
+        return cycle_blk(h, 0, ld, z, r, c, false, dot);
     }
 }

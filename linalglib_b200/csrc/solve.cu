@@ -1214,23 +1214,6 @@ namespace lab
     // last CTA of a segment (per-segment ticket) reducing the K partials in order
     // -- deterministic, and a converged segment is skipped (convergence mask).
     constexpr int kSegK = 8;
-    enum
-    {
-        G_GAMMA = 0,
-        G_PQ    = 1,
-        G_RN    = 2,
-        G_R0    = 3,
-        G_GNEW  = 4,
-        G_N     = 8
-    };
-    enum
-    {
-        GF_DONE   = 0,
-        GF_ITER   = 1,
-        GF_CONV   = 2,
-        GF_STATUS = 3,
-        GF_N      = 4
-    };
     // global flags: [0] = all done, [1] = active segments, [2] = max_iter,
     // [3] = passes of the device-side iteration loop
     struct seg_ws
@@ -1418,7 +1401,6 @@ namespace lab
         precond_impl* M     = nullptr;
         int           multi = 0; // 0: stacked systems, 1: nseg columns of one matrix
         int64_t       n     = 0; // rows of A (multi-RHS column length)
-        int           block = 0; // multi-RHS: block V-cycle over up to 8 columns per pass
     };
 
     static lab_status seg_apply_A(const seg_ops& o, seg_ws& w, const double* in, double* out,
@@ -1446,11 +1428,6 @@ namespace lab
     {
         if(!o.multi)
             return precond_apply(o.M, r, z, s, skip, red_buf());
-        if(o.block)
-        {
-            cyc_ctx c{&o.M->o, s, skip};
-            return cycle_precond_block(o.M->h, c, w.nseg, r, o.n, z, o.n);
-        }
         for(int c = 0; c < w.nseg; c++)
             LAB_TRY(precond_apply(o.M, r + (int64_t)c * o.n, z + (int64_t)c * o.n, s, skip,
                                   red_buf()));
@@ -1673,6 +1650,133 @@ namespace lab
             info->solve_ms         = ms;
             info->status           = status;
         }
+        return status;
+    }
+
+    // ================================================================ block PCG
+    // Up to kBlkMax right-hand sides of one matrix at a time, every vector in the
+    // interleaved block layout (cycle_blk.cu); the recurrences and stopping tests per
+    // column are seg_solve's.  Columns between ncols and ld are zero and retire at once.
+    static lab_status blk_solve(lab_csr_impl* A, precond_impl* M, int ncols, const double* B,
+                                double* X, const lab_iter_control* ctl, int* iters_h, int* conv_h,
+                                lab_solve_info* info, cudaStream_t s)
+    {
+        const int64_t n  = A->m;
+        const int     ld = (ncols + 1) / 2 * 2;
+        LAB_TRY(cycle_prepare_block(M->h, ld, s));
+        dbuf<double>       x, r, z, p, q, sc, partial;
+        dbuf<int>          sf, gflags;
+        dbuf<unsigned int> counter;
+        for(dbuf<double>* v : {&x, &r, &z, &p, &q})
+            LAB_TRY(v->alloc((size_t)n * ld + 2, s));
+        LAB_TRY(sc.alloc((size_t)ld * G_N, s));
+        LAB_TRY(sf.alloc((size_t)ld * GF_N, s));
+        LAB_TRY(gflags.alloc(4, s));
+        LAB_TRY(partial.alloc((size_t)kBlkRedGrid * ld, s));
+        LAB_TRY(counter.alloc(1, s));
+        LAB_CUDA(cudaMemsetAsync(counter.get(), 0, sizeof(unsigned int), s));
+        LAB_CUDA(cudaMemsetAsync(gflags.get(), 0, sizeof(int) * 4, s));
+        LAB_CUDA(cudaMemsetAsync(sf.get(), 0, sizeof(int) * ld * GF_N, s));
+        // one partial buffer and counter serve every reduction: the passes of a solve
+        // run one after another
+        auto red = [&](int slot, const int* skip) {
+            return blk_red{partial.get(), counter.get(), sc.get() + slot, G_N, skip};
+        };
+        const int* skip = gflags.get();
+
+        cudaEvent_t t0, t1;
+        cudaEventCreate(&t0);
+        cudaEventCreate(&t1);
+        cudaEventRecord(t0, s);
+        cudaGraphExec_t gexec  = nullptr;
+        cudaStream_t    cap    = nullptr;
+        int             passes = 0;
+        auto            run    = [&]() -> lab_status {
+            // r = b - A x, r0 = ||r||, z = M r, gamma = (z, r), p = z
+            LAB_TRY(blk_from_columns(X, n, n, ncols, ld, x.get(), s));
+            LAB_TRY(blk_from_columns(B, n, n, ncols, ld, q.get(), s));
+            LAB_TRY(blk_residual(A, ld, x.get(), q.get(), r.get(), s));
+            LAB_TRY(blk_norm(n, ld, r.get(), red(G_R0, nullptr), s));
+            cyc_ctx c0{&M->o, s, nullptr};
+            LAB_TRY(cycle_precond_block(M->h, c0, ld, r.get(), z.get(), red(G_GNEW, nullptr)));
+            LAB_CUDA(cudaMemcpyAsync(p.get(), z.get(), sizeof(double) * n * ld,
+                                     cudaMemcpyDeviceToDevice, s));
+            LAB_TRY(blk_init(sc.get(), sf.get(), gflags.get(), ld, ctl->max_iter, s));
+            LAB_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+            auto iteration = [&](cudaStream_t c) -> lab_status {
+                LAB_TRY(blk_spmv_dot(A, ld, p.get(), q.get(), red(G_PQ, skip), c));
+                LAB_TRY(blk_update(n, ld, x.get(), r.get(), p.get(), q.get(), sc.get(), sf.get(),
+                                   gflags.get(), red(G_RN, skip), ctl->rel_tol, ctl->abs_tol, c));
+                cyc_ctx cc{&M->o, c, skip};
+                LAB_TRY(cycle_precond_block(M->h, cc, ld, r.get(), z.get(), red(G_GNEW, skip)));
+                return blk_pupdate(n, ld, p.get(), z.get(), sc.get(), sf.get(), gflags.get(),
+                                   counter.get(), c);
+            };
+            // one graph launch for all iterations; where conditional nodes are
+            // unavailable the host launches the passes and reads the done flag
+            const int     limit = ctl->max_iter + 1;
+            const int64_t l0    = g_launches.load();
+            int64_t       nodes = 0;
+            lab_status    st = build_loop_graph(cap, gflags.get(), gflags.get() + 3, limit, iteration,
+                                                &gexec, &nodes);
+            if(st == LAB_OK)
+            {
+                // launches counted while capturing are counted again as they run
+                g_launches.fetch_sub(g_launches.load() - l0);
+                LAB_CUDA(cudaGraphLaunch(gexec, s));
+                LAB_TRY(copy_d2h_sync(&passes, gflags.get() + 3, sizeof(int), s));
+                g_launches.fetch_add(1 + (int64_t)passes * nodes);
+            }
+            else if(st == LAB_NOT_SUPPORTED)
+            {
+                for(int it = 0; it < limit; it++)
+                {
+                    LAB_TRY(iteration(s));
+                    int done = 0;
+                    LAB_TRY(copy_d2h_sync(&done, gflags.get(), sizeof(int), s));
+                    if(done)
+                        break;
+                }
+            }
+            else
+                return st;
+            return blk_to_columns(x.get(), n, ncols, ld, X, n, s);
+        };
+        lab_status st = run();
+        cudaEventRecord(t1, s);
+        cudaStreamSynchronize(s);
+        float ms = 0.f;
+        cudaEventElapsedTime(&ms, t0, t1);
+        std::vector<int> f((size_t)ld * GF_N);
+        if(st == LAB_OK)
+            st = copy_d2h_sync(f.data(), sf.get(), sizeof(int) * f.size(), s);
+        if(gexec)
+            cudaGraphExecDestroy(gexec);
+        if(cap)
+            cudaStreamDestroy(cap);
+        cudaEventDestroy(t0);
+        cudaEventDestroy(t1);
+        LAB_TRY(st);
+        int maxit = 0, allconv = 1, nan = 0;
+        for(int k = 0; k < ncols; k++)
+        {
+            if(iters_h)
+                iters_h[k] = f[k * GF_N + GF_ITER];
+            if(conv_h)
+                conv_h[k] = f[k * GF_N + GF_CONV];
+            maxit = std::max(maxit, f[k * GF_N + GF_ITER]);
+            allconv &= f[k * GF_N + GF_CONV];
+            nan |= f[k * GF_N + GF_STATUS] == LAB_NAN;
+        }
+        const lab_status status = allconv ? LAB_OK : (nan ? LAB_NAN : LAB_NOT_CONVERGED);
+        if(status == LAB_NAN)
+            set_error("segmented pcg: a system's residual became NaN/Inf");
+        info->iterations       = maxit;
+        info->converged        = allconv;
+        info->initial_residual = 0.0;
+        info->final_residual   = 0.0;
+        info->solve_ms         = ms;
+        info->status           = status;
         return status;
     }
 }
@@ -2051,6 +2155,35 @@ LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, c
     LAB_TRY(spmv_analyse(A, s));
     if(M->kind == 0)
         LAB_TRY(cycle_prepare(M->h, &M->o, s));
+    if(M->kind == 0 && cycle_block_supported(M->h, &M->o) && M->h->A[0]->m == A->m)
+    {
+        // as few blocks as kBlkMax allows, of about equal size
+        const int      nblk = (int)ceil_div<int64_t>(nrhs, kBlkMax);
+        const int      per  = (int)ceil_div<int64_t>(nrhs, nblk);
+        lab_solve_info all{};
+        lab_status     worst = LAB_OK;
+        all.converged        = 1;
+        for(int k = 0; k < nrhs; k += per)
+        {
+            lab_solve_info   one{};
+            const int        nc = std::min(per, nrhs - k);
+            const lab_status st =
+                blk_solve(A, M, nc, B + (int64_t)k * A->m, X + (int64_t)k * A->m, c,
+                          iterations ? iterations + k : nullptr, converged ? converged + k : nullptr,
+                          &one, s);
+            if(st != LAB_OK && st != LAB_NOT_CONVERGED && st != LAB_NAN)
+                return st;
+            if(st == LAB_NAN || worst == LAB_OK)
+                worst = st;
+            all.iterations = std::max(all.iterations, one.iterations);
+            all.converged &= one.converged;
+            all.solve_ms += one.solve_ms;
+        }
+        all.status = worst;
+        if(info)
+            *info = all;
+        return worst;
+    }
     std::vector<int64_t> off((size_t)nrhs + 1);
     for(int k = 0; k <= nrhs; k++)
         off[k] = (int64_t)k * A->m;
@@ -2059,11 +2192,6 @@ LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, c
     o.M     = M;
     o.multi = 1;
     o.n     = A->m;
-    if(M->kind == 0 && cycle_block_supported(M->h, &M->o))
-    {
-        LAB_TRY(cycle_prepare_block(M->h, s));
-        o.block = 1;
-    }
     return seg_solve(o, nrhs, off.data(), B, X, c, iterations, converged, info, s);
 }
 

@@ -1,0 +1,47 @@
+"""Block PCG over interleaved columns (csrc/cycle_blk.cu) at odd and even column counts,
+one and two blocks, short and long rows, a zero column and a nonzero guess, against the
+oracle's PCG column by column."""
+import numpy as np
+import pytest
+
+from linalglib_b200 import _lib as L
+from linalglib_b200 import problems as P
+
+pytestmark = pytest.mark.gpu
+
+OPS = {"2d 31x40": lambda: P.poisson2d(31, 40), "3d 12": lambda: P.poisson3d(12),
+       "27pt 9": lambda: P.diffusion27(9)}
+
+
+@pytest.mark.parametrize("n1, n2", [(1, 1), (2, 2)])
+@pytest.mark.parametrize("ncols", [1, 2, 5, 32, 65])
+@pytest.mark.parametrize("op", list(OPS))
+def test_block_pcg(gpu, oracle, op, ncols, n1, n2):
+    A = OPS[op]()
+    m = A[0].size - 1
+    rng = np.random.default_rng(ncols)
+    B = np.stack([P.csr_matvec(*A, rng.uniform(-1, 1, m)) for _ in range(ncols)])
+    X0 = np.zeros((ncols, m))
+    if ncols > 2:
+        B[1] = 0.0
+        X0[2] = rng.uniform(-1, 1, m)
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    M = gpu.Preconditioner.amg(gpu.Hierarchy(dA, kind=L.AMG_SA),
+                               gpu.amg_options(n1=n1, n2=n2, omega=2.0 / 3.0))
+    X, iters, conv, info = gpu.multi_rhs_pcg(
+        dA, gpu.vec(B).reshape(ncols, m), M, X=gpu.vec(X0).reshape(ncols, m),
+        control=gpu.iter_control(rel_tol=1e-9, abs_tol=0.0))
+    assert info.converged == 1 and np.all(conv == 1)
+    X = X.cpu().numpy()
+    H = oracle.amg_setup(A, kind=0)
+    for k in range(min(ncols, 6)):
+        if k == 1 and ncols > 2:
+            assert iters[k] == 0 and np.all(X[k] == 0.0)
+            continue
+        xo, it, _ = H.pcg(B[k], x0=X0[k], n1=n1, n2=n2, omega=2.0 / 3.0, coarse=1, rel_tol=1e-9)
+        assert abs(int(iters[k]) - it) <= 1
+        # both stop at a relative residual of 1e-9; condition numbers are below 1e4
+        assert np.max(np.abs(X[k] - xo)) <= 1e-5 * np.max(np.abs(xo))
+    for k in range(ncols):
+        r = B[k] - P.csr_matvec(*A, X[k])
+        assert np.max(np.abs(r)) <= 2e-9 * max(np.max(np.abs(B[k] - P.csr_matvec(*A, X0[k]))), 1e-30)

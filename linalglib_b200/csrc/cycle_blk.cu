@@ -16,7 +16,7 @@
 // Measured, 32 right-hand sides on a 64^3 Poisson system: groups of 8 columns, one
 // thread per row with 8 accumulators and conversions to and from the block layout
 // around every cycle, 55.6 ms (120 launches and 2 ms an iteration; a warp's 16-byte
-// load of 32 separate rows is 32 lookups); this layout 28.6 ms.
+// load of 32 separate rows is 32 lookups); this layout 25.1 ms.
 #include "cycle.cuh"
 
 #include <algorithm>
@@ -244,10 +244,14 @@ namespace lab
 
     // ------------------------------------------------------------ row kernel
     // Threads of a CTA: (row slot, part of the row, column pair), the pair fastest.
+    // Four CTAs per SM, one wave: at the 80 registers that the compiler takes without a
+    // bound only three fit, and a grid of four per SM ran a second wave a third full
+    // (32 right-hand sides on 64^3: 28.6 -> 25.1 ms; consecutive rows per CTA instead
+    // of a grid stride: 25.6).
     // The next entries' columns and values are loaded while the gathers of the
     // current ones are in flight.
     template <class Op, class IT>
-    __global__ void __launch_bounds__(kBlkNT)
+    __global__ void __launch_bounds__(kBlkNT, 4)
         k_blk_rows(csr_view<double, IT> A, Op op, int kl, int W, blk_red red)
     {
         constexpr int U = 4;
@@ -353,8 +357,8 @@ namespace lab
               A->nnz >= 8 * A->m * W)
             W *= 2;
         const int64_t  per  = kBlkNT / (kl * W);
-        const unsigned grid = (unsigned)std::min<int64_t>(
-            ceil_div<int64_t>(A->m, per), Op::kDot ? kBlkRedGrid : (int64_t)num_sms() * 32);
+        const unsigned grid =
+            (unsigned)std::min<int64_t>(ceil_div<int64_t>(A->m, per), kBlkRedGrid);
         if(A->lp.dcol)
         {
             csr_view<double, int16_t> V{A->row_ptr, A->lp.dcol, A->val, (int32_t)A->m};

@@ -2,9 +2,9 @@
 // the reference's csrtrsv / csrilu0 / csric0 and its ILU(0), IC(0), Gauss-Seidel
 // and SOR preconditioners.
 //
-// Rows are grouped into dependency levels once per matrix pattern (on the host:
-// a row's level is one more than the deepest row it reads).  A solve is one
-// launch (after one that marks x pending): warps claim 32-row chunks in level
+// Rows are grouped into dependency levels once per matrix pattern (a row's level
+// is one more than the deepest row it reads).  A solve is one launch (after one that
+// marks a copy of x, in level order, pending): warps claim 32-row chunks in level
 // order from an atomic counter, and each lane walks its row in the reference's
 // order, reading a dependency once its value is no longer marked pending.  A
 // chunk only waits on rows claimed before it, by warps that are running, so
@@ -27,6 +27,15 @@ namespace lab
     {
         std::vector<int> ptr;          // level k: rows[ptr[k] .. ptr[k+1])
         int32_t*         rows = nullptr; // device, rows ordered by level
+        // the solve's view of the triangle (device): the entries the reference's
+        // loop visits in rows[t], in its order, are [ent_ptr[t], ent_ptr[t + 1]);
+        // col is the place of the entry's column in rows[], or kTriDiag
+        int32_t* ent_ptr = nullptr;
+        int32_t* ent_col = nullptr;
+        int32_t* ent_src = nullptr; // position of the entry's value in the matrix
+        int32_t* gate    = nullptr; // per 32 rows: a place solved two levels earlier, or -1
+        double*  x       = nullptr; // the solution in the order of rows[]
+        int      longest = 0;       // entries of the longest row
     };
 
     struct tri_plan
@@ -46,10 +55,11 @@ namespace lab
     {
         if(!A->tri)
             return;
-        if(A->tri->lower.rows)
-            cudaFree(A->tri->lower.rows);
-        if(A->tri->upper.rows)
-            cudaFree(A->tri->upper.rows);
+        for(tri_sched* t : {&A->tri->lower, &A->tri->upper})
+            for(void* p : {(void*)t->rows, (void*)t->ent_ptr, (void*)t->ent_col,
+                           (void*)t->ent_src, (void*)t->gate, (void*)t->x})
+                if(p)
+                    cudaFree(p);
         if(A->tri->diag)
             cudaFree(A->tri->diag);
         if(A->tri->ctl)
@@ -350,6 +360,106 @@ namespace lab
         return order_levels(out, lptr.get(), m, hc.nlev, s);
     }
 
+    // ------------------------------------------------------------ solve layout
+    constexpr int kTriDiag = -1; // ent_col of the diagonal
+
+    __global__ void k_tri_place(const int32_t* __restrict__ order, int m, int32_t* __restrict__ place)
+    {
+        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+        if(t < m)
+            place[order[t]] = t;
+    }
+
+    // The entries the reference visits in row i, in its order: forward
+    // (host_csrtrsv.cpp:36-64) the row up to the first column right of the diagonal,
+    // backward (66-90) the row right to left without the columns left of it.
+    // FILL false: their number; true: their columns' places and value positions.
+    template <bool LOWER, bool FILL>
+    __global__ void k_tri_entries(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+                                  const int32_t* __restrict__ order,
+                                  const int32_t* __restrict__ place, int m, int32_t* ent_ptr,
+                                  int32_t* __restrict__ ent_col, int32_t* __restrict__ ent_src,
+                                  int* longest)
+    {
+        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+        if(t >= m)
+            return;
+        const int i = order[t], a = rp[i], e = rp[i + 1];
+        int       n = FILL ? ent_ptr[t] : 0;
+        const int n0 = n;
+        for(int k = 0; k < e - a; k++)
+        {
+            const int j = LOWER ? a + k : e - 1 - k;
+            const int c = ci[j];
+            if(LOWER ? c > i : c < i)
+            {
+                if(LOWER)
+                    break;
+                continue;
+            }
+            if(FILL)
+            {
+                ent_col[n] = c == i ? kTriDiag : place[c];
+                ent_src[n] = j;
+            }
+            n++;
+        }
+        if(!FILL)
+        {
+            ent_ptr[t] = n - n0;
+            if(n - n0 > *(volatile int*)longest)
+                atomicMax(longest, n - n0);
+        }
+    }
+
+    // For the chunk of 32 rows that starts at row t0: the dependency nearest in the
+    // order of the nearest dependency of row t0, -1 if there is none.
+    __global__ void k_tri_gate(const int32_t* __restrict__ ent_ptr,
+                               const int32_t* __restrict__ ent_col, int m,
+                               int32_t* __restrict__ gate)
+    {
+        const int w = blockIdx.x * blockDim.x + threadIdx.x;
+        if(w >= ceil_div(m, 32))
+            return;
+        int g = w * 32;
+        for(int up = 0; up < 2 && g >= 0; up++)
+        {
+            int far = -1;
+            for(int j = ent_ptr[g]; j < ent_ptr[g + 1]; j++)
+                far = max(far, ent_col[j]);
+            g = far;
+        }
+        gate[w] = g;
+    }
+
+    static lab_status tri_layout(const lab_csr_impl* A, bool lower, tri_sched& t, cudaStream_t s)
+    {
+        const int      m = (int)A->m;
+        const unsigned g = (unsigned)ceil_div(m, 256);
+        dbuf<int32_t>  place;
+        dbuf<int>      longest;
+        int64_t        n = 0;
+        LAB_TRY(place.alloc((size_t)m, s));
+        LAB_TRY(longest.alloc(1, s));
+        LAB_CUDA(cudaMemsetAsync(longest.get(), 0, sizeof(int), s));
+        LAB_TRY(dalloc(&t.ent_ptr, (size_t)m + 1, s));
+        LAB_LAUNCH(k_tri_place, g, 256, 0, s, (const int32_t*)t.rows, m, place.get());
+        LAB_LAUNCH((lower ? k_tri_entries<true, false> : k_tri_entries<false, false>), g, 256, 0, s,
+                   A->row_ptr, A->col_ind, (const int32_t*)t.rows, (const int32_t*)place.get(), m,
+                   t.ent_ptr, (int32_t*)nullptr, (int32_t*)nullptr, longest.get());
+        LAB_TRY(counts_to_rowptr(t.ent_ptr, t.ent_ptr, m, &n, s));
+        LAB_TRY(dalloc(&t.ent_col, (size_t)std::max<int64_t>(n, 1), s));
+        LAB_TRY(dalloc(&t.ent_src, (size_t)std::max<int64_t>(n, 1), s));
+        LAB_TRY(dalloc(&t.gate, (size_t)ceil_div(m, 32), s));
+        LAB_TRY(dalloc(&t.x, (size_t)m, s));
+        LAB_LAUNCH((lower ? k_tri_entries<true, true> : k_tri_entries<false, true>), g, 256, 0, s,
+                   A->row_ptr, A->col_ind, (const int32_t*)t.rows, (const int32_t*)place.get(), m,
+                   t.ent_ptr, t.ent_col, t.ent_src, longest.get());
+        LAB_LAUNCH(k_tri_gate, (unsigned)ceil_div(ceil_div(m, 32), 256), 256, 0, s,
+                   (const int32_t*)t.ent_ptr, (const int32_t*)t.ent_col, m, t.gate);
+        return copy_d2h_sync(&t.longest, longest.get(), sizeof(int), s);
+    }
+
     lab_status tri_analyse(lab_csr_impl* A, cudaStream_t s)
     {
         if(A->tri)
@@ -377,6 +487,10 @@ namespace lab
             st = level_sched_dev(A, true, p->lower, s);
         if(st == LAB_OK && m > 0)
             st = level_sched_dev(A, false, p->upper, s);
+        if(st == LAB_OK && m > 0)
+            st = tri_layout(A, true, p->lower, s);
+        if(st == LAB_OK && m > 0)
+            st = tri_layout(A, false, p->upper, s);
         if(st == LAB_OK)
             st = dalloc(&p->ctl, 2, s);
         if(st == LAB_OK && cudaMemsetAsync(p->ctl, 0, sizeof(int32_t) * 2, s) != cudaSuccess)
@@ -391,15 +505,14 @@ namespace lab
     }
 
     // ------------------------------------------------------------ solves
-    // x is filled with kTriPending before a solve and every x_i is written once,
-    // by the row's lane, as the result of a double operation.  Such a result is
-    // never a signalling NaN (arithmetic returns a quiet NaN), so a value other
-    // than kTriPending is the solved x_i: the value is its own "solved" flag and
-    // a dependency costs one L2 round trip (relaxed 64-bit loads and stores at
+    // tri_sched::x is filled with kTriPending before a solve and every entry is
+    // written once, by the row's lane, as the result of a double operation.  Such a
+    // result is never a signalling NaN (arithmetic returns a quiet NaN), so a value
+    // other than kTriPending is the solved one: the value is its own "solved" flag
+    // and a dependency costs one L2 round trip (relaxed 64-bit loads and stores at
     // GPU scope, single-copy atomic).
     constexpr uint64_t kTriPending = 0x7ff4d1b0c0de0001ull; // signalling NaN
     constexpr int      kTriBlock   = 256;
-    constexpr int      kTriPf      = 8;        // entries of a row held in registers
     constexpr unsigned kTriIdle    = 1u << 26; // default idle rounds before a warp gives up
 
     __device__ __forceinline__ uint64_t ld_relaxed(const double* p)
@@ -431,49 +544,39 @@ namespace lab
             *counter = 0;
     }
 
-    // One entry of a lane's row, in the reference's order, given the entry's
-    // dependency value xv (kTriPending: not solved yet -> false).  LOWER,
-    // host_forward_solve_impl (host_csrtrsv.cpp:36-64): fma over the entries left
-    // of the diagonal in CSR order, stop at the first entry right of it (or at the
-    // diagonal when unit); dscale != 0 scales the diagonal (SOR_precond's M,
-    // preconditioner.cpp:137-147).  Upper, host_backward_solve_impl (66-90): walk
-    // the row right to left subtracting a_ij x_j (multiply, then subtract), keep
-    // the diagonal.
-    template <bool LOWER>
-    __device__ __forceinline__ bool tri_entry(int c, double a, uint64_t xv, int i, int unit,
-                                              double dscale, int len, int& k, double& acc,
-                                              double& d)
-    {
-        if(LOWER ? c < i : c > i)
-        {
-            if(xv == kTriPending)
-                return false;
-            const double xc = __longlong_as_double((long long)xv);
-            acc             = LOWER ? fma(a, xc, acc) : __dsub_rn(acc, __dmul_rn(a, xc));
-            k++;
-        }
-        else if(c == i && !unit)
-        {
-            d = (LOWER && dscale != 0.0) ? __dmul_rn(a, dscale) : a;
-            k++;
-        }
-        else
-            k = LOWER ? len : k + 1; // the forward loop breaks here
-        return true;
-    }
-
-    // Warps claim 32-row chunks of `order` (rows by level) from ctl[0]; each lane
-    // polls the dependencies of its row's next entries at once, consumes the solved
-    // prefix in order, and writes x_i when the row is done.  ctl[1] is the error
-    // flag, set when a warp waited idle_limit rounds without progress; the other
-    // warps see it when they claim their next chunk or every 1024 idle rounds and
-    // return.  held (>= 0) is a row whose value is never written: the rows that
-    // depend on it can only run out of their wait (the test of this path).
-    template <bool LOWER>
+    // Warps claim chunks of 32 consecutive rows of the level order from ctl[0].  A
+    // lane holds PF entries of its row (place of the column, value) in registers,
+    // polls the pending ones all at once, and when they are there walks them in the
+    // reference's order, the next PF entries after that, and writes the row's value.
+    // LOWER, host_forward_solve_impl (host_csrtrsv.cpp:36-64): fma over the entries
+    // left of the diagonal in CSR order, stop at the diagonal when unit; dscale != 0
+    // scales the diagonal (SOR_precond's M, preconditioner.cpp:137-147).  Upper,
+    // host_backward_solve_impl (66-90): walk the row right to left subtracting
+    // a_ij x_j (multiply, then subtract), keep the diagonal.
+    //
+    // Bound by the chain of levels: store -> L2 -> poll -> arithmetic, per level.
+    // What keeps that chain short:
+    //  - x is polled in level order, where the 32 rows of a chunk read nearly
+    //    consecutive places of the level before (in row order each poll of a warp
+    //    touched up to 32 sectors per entry, 1 GB of L2 reads a solve at 64^3);
+    //  - a warp whose chunk is more than a level ahead polls one word only, its gate
+    //    (two levels earlier), so the polls of the level that is being solved do not
+    //    queue behind those of a dozen later ones;
+    //  - no sleep between the polls of the level that is next.
+    // ILU(0)-PCG, 64^3 7-point: 41.7 -> 28.9 ms; 100^2 5-point 43.7 -> 29.4 ms (polls in
+    // row order, of every outstanding entry, by every warp -> this).
+    //
+    // ctl[1] is the error flag, set when a warp waited idle_limit rounds without
+    // progress; the other warps see it when they claim their next chunk or every
+    // 1024 idle rounds and return.  held (>= 0) is a row whose value is never
+    // written: the rows that depend on it can only run out of their wait (the test
+    // of this path).
+    template <bool LOWER, int PF>
     __global__ void __launch_bounds__(kTriBlock)
-        k_trsv(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
+        k_trsv(const int32_t* __restrict__ ent_ptr, const int32_t* __restrict__ ent_col,
+               const int32_t* __restrict__ ent_src, const int32_t* __restrict__ gate,
                const double* __restrict__ v, const int32_t* __restrict__ order, int m, int unit,
-               double dscale, const double* __restrict__ b, double* x, int32_t* ctl,
+               double dscale, const double* b, double* x, double* xl, int32_t* ctl,
                const int* skip, unsigned idle_limit, int held)
     {
         if(skip && *skip)
@@ -489,67 +592,96 @@ namespace lab
                 return;
             const int t    = base + lane;
             bool      done = t >= m;
-            int       i = 0, a = 0, e = 0, len = 0, k = 0;
+            int       i = 0, k = 0, e = 0;
             double    acc = 0.0, d = 1.0, bi = 0.0;
-            int       pc[kTriPf];
-            double    pv[kTriPf];
+            int       pc[PF];
+            double    pv[PF];
+            uint64_t  xv[PF];
+            unsigned  need = 0;
+            auto      hold = [&]() { // entries k .. k + PF of the row
+                need = 0;
+#pragma unroll
+                for(int q = 0; q < PF; q++)
+                {
+                    const bool ok = k + q < e;
+                    pc[q]         = ok ? ent_col[k + q] : kTriDiag;
+                    pv[q]         = ok ? v[ent_src[k + q]] : 0.0;
+                    xv[q]         = 0;
+                    need |= (unsigned)(pc[q] >= 0) << q;
+                }
+            };
             if(!done)
             {
-                i   = order[t];
-                a   = rp[i];
-                e   = rp[i + 1];
-                len = e - a;
-#pragma unroll
-                for(int q = 0; q < kTriPf; q++)
-                {
-                    const int j = LOWER ? a + q : e - 1 - q;
-                    pc[q]       = q < len ? ci[j] : i;
-                    pv[q]       = q < len ? v[j] : 0.0;
-                }
+                i = order[t];
+                k = ent_ptr[t];
+                e = ent_ptr[t + 1];
+                hold();
                 if(LOWER)
                     bi = b[i];
                 else
                     acc = b[i];
             }
-            unsigned idle = 0;
+            const int g    = gate[base >> 5];
+            unsigned  idle = 0;
+            bool      far  = g >= 0;
             for(;;)
             {
                 bool progress = false;
-                if(!done)
+                if(far)
                 {
-                    const int k0 = k;
-                    // all outstanding dependencies of the held entries in flight at once
-                    uint64_t xv[kTriPf];
+                    far      = ld_relaxed(xl + g) == kTriPending;
+                    progress = !far;
+                }
+                else if(!done)
+                {
+                    uint64_t u[PF];
 #pragma unroll
-                    for(int q = 0; q < kTriPf; q++)
-                        xv[q] = (q >= k && q < len && (LOWER ? pc[q] < i : pc[q] > i))
-                                    ? ld_relaxed(x + pc[q])
-                                    : 0;
-                    bool blocked = false;
+                    for(int q = 0; q < PF; q++)
+                        u[q] = (need >> q & 1u) ? ld_relaxed(xl + pc[q]) : kTriPending;
 #pragma unroll
-                    for(int q = 0; q < kTriPf; q++)
-                        if(!blocked && q == k && k < len)
-                            blocked = !tri_entry<LOWER>(pc[q], pv[q], xv[q], i, unit, dscale, len,
-                                                        k, acc, d);
-                    while(!blocked && k < len) // entries beyond the held ones
+                    for(int q = 0; q < PF; q++)
+                        if(u[q] != kTriPending)
+                        {
+                            xv[q] = u[q];
+                            need &= ~(1u << q);
+                            progress = true;
+                        }
+                    if(need == 0)
                     {
-                        const int j  = LOWER ? a + k : e - 1 - k;
-                        const int c  = ci[j];
-                        uint64_t  xc = (LOWER ? c < i : c > i) ? ld_relaxed(x + c) : 0;
-                        blocked = !tri_entry<LOWER>(c, v[j], xc, i, unit, dscale, len, k, acc, d);
-                    }
-                    progress = k != k0;
-                    if(!blocked && i == held)
-                    {
-                        done     = true; // x_i stays pending
+                        bool stop = false;
+#pragma unroll
+                        for(int q = 0; q < PF; q++)
+                        {
+                            if(stop || k + q >= e)
+                                continue;
+                            if(pc[q] >= 0)
+                            {
+                                const double xc = __longlong_as_double((long long)xv[q]);
+                                acc = LOWER ? fma(pv[q], xc, acc)
+                                            : __dsub_rn(acc, __dmul_rn(pv[q], xc));
+                            }
+                            else if(!unit)
+                                d = (LOWER && dscale != 0.0) ? __dmul_rn(pv[q], dscale) : pv[q];
+                            else
+                                stop = LOWER;
+                        }
+                        k += PF;
                         progress = true;
-                    }
-                    else if(!blocked)
-                    {
-                        st_relaxed(x + i,
-                                   LOWER ? __ddiv_rn(__dsub_rn(bi, acc), d) : __ddiv_rn(acc, d));
-                        done     = true;
-                        progress = true;
+                        if(!stop && k < e)
+                            hold();
+                        else
+                        {
+                            done = true;
+                            if(i != held) // else its value stays pending
+                            {
+                                // (a - b) / 1 is a - b
+                                double r = LOWER ? __dsub_rn(bi, acc) : acc;
+                                if(!LOWER || !unit)
+                                    r = __ddiv_rn(r, d);
+                                st_relaxed(xl + t, r);
+                                x[i] = r;
+                            }
+                        }
                     }
                 }
                 if(__all_sync(0xffffffffu, done))
@@ -566,18 +698,32 @@ namespace lab
                     }
                     if((idle & 1023u) == 0 && __any_sync(0xffffffffu, ld_acquire(ctl + 1) != 0))
                         return;
-                    __nanosleep(idle < 8 ? 0 : 64);
+                    if(far)
+                        __nanosleep(32);
                 }
             }
         }
     }
 
-    // One CTA (8 warps) per SM: 37,888 rows in flight on 148 SMs, more than the
-    // widest level of the 128^3 7-point solve; more warps only add polling traffic
-    // (measured: 740 us per 128^3 solve at 1 CTA per SM, 860 us at 3).
+    // One CTA (8 warps) per SM: 37,888 rows in flight on 148 SMs, a dozen levels of the
+    // 64^3 7-point solve ahead (ILU(0)-PCG on it: 28.9 ms with 1 CTA per SM, 29.4 with
+    // 2, 30.4 with 4; 100^2 5-point: 29.4 ms with each).
     static int trsv_grid(int m)
     {
         return (int)std::max<int64_t>(1, std::min<int64_t>(num_sms(), ceil_div(m, kTriBlock)));
+    }
+
+    template <bool LOWER, int PF>
+    static lab_status trsv_launch(const lab_csr_impl* A, const tri_plan& p, const tri_sched& t,
+                                  bool unit, double dscale, const double* b, double* x,
+                                  cudaStream_t s, const int* skip)
+    {
+        const int m = (int)A->m;
+        LAB_LAUNCH((k_trsv<LOWER, PF>), trsv_grid(m), kTriBlock, 0, s, (const int32_t*)t.ent_ptr,
+                   (const int32_t*)t.ent_col, (const int32_t*)t.ent_src, (const int32_t*)t.gate,
+                   (const double*)A->val, (const int32_t*)t.rows, m, (int)unit, dscale, b, x, t.x,
+                   p.ctl, skip, p.idle_limit ? p.idle_limit : kTriIdle, p.held_row);
+        return LAB_OK;
     }
 
     lab_status tri_solve(lab_csr_impl* A, bool lower, bool unit, double dscale, const double* b,
@@ -586,9 +732,10 @@ namespace lab
         if(A->m == 0)
             return LAB_OK;
         LAB_TRY(tri_analyse(A, s));
-        tri_plan& p = *A->tri;
-        const int m = (int)A->m;
-        if(b < x + m && x < b + m) // in place: x is overwritten by the pending marks first
+        tri_plan&        p = *A->tri;
+        const tri_sched& t = lower ? p.lower : p.upper;
+        const int        m = (int)A->m;
+        if(b < x + m && x < b + m && b != x) // overlapping: rows would read what others wrote
         {
             if(!p.scratch)
                 LAB_TRY(dalloc(&p.scratch, (size_t)m, s));
@@ -596,17 +743,13 @@ namespace lab
             b = p.scratch;
         }
         LAB_LAUNCH(k_trsv_prep, (unsigned)std::min<int64_t>(ceil_div(m, 256), 4 * num_sms()), 256,
-                   0, s, x, m, p.ctl, skip);
-        const unsigned idle = p.idle_limit ? p.idle_limit : kTriIdle;
+                   0, s, t.x, m, p.ctl, skip);
+        // 4 held entries cover a triangle of a 5- or 7-point operator with its diagonal
         if(lower)
-            LAB_LAUNCH(k_trsv<true>, trsv_grid(m), kTriBlock, 0, s, A->row_ptr, A->col_ind,
-                       (const double*)A->val, (const int32_t*)p.lower.rows, m, (int)unit, dscale,
-                       b, x, p.ctl, skip, idle, p.held_row);
-        else
-            LAB_LAUNCH(k_trsv<false>, trsv_grid(m), kTriBlock, 0, s, A->row_ptr,
-                       A->col_ind, (const double*)A->val, (const int32_t*)p.upper.rows, m,
-                       (int)unit, 0.0, b, x, p.ctl, skip, idle, p.held_row);
-        return LAB_OK;
+            return t.longest <= 4 ? trsv_launch<true, 4>(A, p, t, unit, dscale, b, x, s, skip)
+                                  : trsv_launch<true, 8>(A, p, t, unit, dscale, b, x, s, skip);
+        return t.longest <= 4 ? trsv_launch<false, 4>(A, p, t, unit, 0.0, b, x, s, skip)
+                              : trsv_launch<false, 8>(A, p, t, unit, 0.0, b, x, s, skip);
     }
 
     lab_status tri_check(lab_csr_impl* A, cudaStream_t s)

@@ -250,3 +250,42 @@ def test_diagonal_scalings_match_reference(gpu, reference, name):
                           [dB.to_numpy()[2][j] for j in
                            [next(k for k in range(A[0][i], A[0][i + 1]) if A[1][k] == i)
                             for i in range(A[0].size - 1)]])
+
+
+def _band(n, k, seed, shuffle):
+    """Rows with up to k columns on each side of the diagonal, among the 40 nearest;
+    shuffle: the columns of a row in any order."""
+    rng = np.random.default_rng(seed)
+    rp, ci, v = [0], [], []
+    for i in range(n):
+        lo, hi = np.arange(max(0, i - 40), i), np.arange(i + 1, min(n, i + 41))
+        cols = np.concatenate([rng.choice(lo, min(k, lo.size), replace=False), [i],
+                               rng.choice(hi, min(k, hi.size), replace=False)]).astype(int)
+        cols = rng.permutation(cols) if shuffle else np.sort(cols)
+        vals = np.where(cols == i, 4.0 * k, rng.uniform(-1, 1, cols.size))
+        ci += cols.tolist()
+        v += vals.tolist()
+        rp.append(len(ci))
+    return np.array(rp, np.int32), np.array(ci, np.int32), np.array(v, np.float64)
+
+
+@pytest.mark.parametrize("shuffle", [False, True])
+@pytest.mark.parametrize("n,k", [(31, 3), (32, 3), (33, 4), (257, 7), (257, 8), (4100, 3),
+                                 (1000, 16)])
+def test_trsv_row_lengths_bit_exact(gpu, oracle, n, k, shuffle):
+    """Rows of at most, of more and of many times the entries a lane holds (4 or 8,
+    the diagonal among them), chunks of 32 rows with a remainder, rows in any column
+    order, and b solved in place."""
+    from linalglib_b200 import _lib as L
+    A = _band(n, k, n + k, shuffle)
+    b = np.random.default_rng(n).uniform(-1, 1, n)
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    for lower in (True, False):
+        for unit in (True, False):
+            want = _bits(oracle.trsv(A, b, lower, unit))
+            x = dA.trsv(gpu.vec(b), lower=lower, unit_diag=unit)
+            assert np.array_equal(_bits(x.cpu().numpy()), want)
+            y = gpu.vec(b)
+            L.call("lab_csrtrsv", dA.h, int(lower), int(unit), gpu.ptr(y), gpu.ptr(y),
+                   gpu.stream_handle())
+            assert np.array_equal(_bits(y.cpu().numpy()), want)

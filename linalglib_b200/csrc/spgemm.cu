@@ -483,13 +483,13 @@ namespace lab
         return slot;
     }
 
-    // MODE 0: symbolic (counts[row], or the row goes to the overflow list when more
-    // than 3/4 of the table fills up); MODE 1: numeric into out_rp / out_ci / out_v.
+    // MODE 0: symbolic (counts[row], or the row goes to the overflow list when it has
+    // more than limit columns); MODE 1: numeric into out_rp / out_ci / out_v.
     template <int MODE, int HS, int WARPS>
     __global__ void __launch_bounds__(32 * WARPS)
         k_hash_gemm(csr_ref A, csr_ref B, const int32_t* __restrict__ rows, int nrows,
                     int32_t* counts, const int32_t* __restrict__ out_rp, int32_t* out_ci,
-                    double* out_v, int32_t* ovf_rows, int* n_ovf, const int* nrows_dev)
+                    double* out_v, int32_t* ovf_rows, int* n_ovf, int limit, const int* nrows_dev)
     {
         if(nrows_dev) // the list's length is known on the device only (nrows: its capacity)
             nrows = min(nrows, *nrows_dev);
@@ -641,7 +641,7 @@ namespace lab
                         }
                         __syncwarp();
                     }
-                    if(MODE == 0 && sm.claims > 3 * HS / 4)
+                    if(MODE == 0 && sm.claims > limit)
                         ovf = true; // too many distinct columns for this table
                 }
                 __syncwarp();
@@ -820,8 +820,8 @@ namespace lab
     template <int MODE, int HS, int WARPS>
     static lab_status launch_hash_cls(csr_ref Ar, csr_ref Br, const int32_t* rows, int n,
                                       int32_t* counts, const int32_t* out_rp, int32_t* out_ci,
-                                      double* out_v, int32_t* ovf_rows, int* n_ovf, cudaStream_t s,
-                                      const int* n_dev = nullptr)
+                                      double* out_v, int32_t* ovf_rows, int* n_ovf, int limit,
+                                      cudaStream_t s, const int* n_dev = nullptr)
     {
         if(n == 0)
             return LAB_OK;
@@ -841,8 +841,16 @@ namespace lab
         const unsigned grid = (unsigned)std::min<int64_t>(ceil_div<int64_t>(n, WARPS),
                                                           (int64_t)num_sms() * occ);
         LAB_LAUNCH((k_hash_gemm<MODE, HS, WARPS>), grid, 32 * WARPS, smem, s, Ar, Br, rows, n,
-                   counts, out_rp, out_ci, out_v, ovf_rows, n_ovf, n_dev);
+                   counts, out_rp, out_ci, out_v, ovf_rows, n_ovf, limit, n_dev);
         return LAB_OK;
+    }
+
+    // Columns a row of the symbolic pass may have in a table of HS slots.  With
+    // slots >= the row's product bound (sym >= 2, tables below 1024) every row fits;
+    // else a row that fills 3/4 is retried with 4096 slots.
+    constexpr int sym_limit(int HS, const gemm_tune& t)
+    {
+        return t.sym >= 2 && HS < 1024 ? HS : 3 * HS / 4;
     }
 
     // One launch per non-empty hash class (1..6) of the phase.
@@ -850,13 +858,13 @@ namespace lab
     static lab_status launch_hash_classes(const gemm_classes& g, csr_ref Ar, csr_ref Br,
                                           int32_t* counts, const int32_t* out_rp, int32_t* out_ci,
                                           double* out_v, int32_t* ovf_rows, int* n_ovf,
-                                          stream_fork& f)
+                                          const gemm_tune& tune, stream_fork& f)
     {
         // the classes are independent row sets: they run side by side
 #define LAB_HASH_CLS(C, HS, W)                                                                    \
     if(g.count(C))                                                                                \
         LAB_TRY((launch_hash_cls<MODE, HS, W>(Ar, Br, g.of(C), g.count(C), counts, out_rp, out_ci,\
-                                              out_v, ovf_rows, n_ovf, f.next())))
+                                              out_v, ovf_rows, n_ovf, sym_limit(HS, tune), f.next())))
         if constexpr(MODE == 0)
         {
             LAB_HASH_CLS(1, 128, 8);
@@ -973,7 +981,11 @@ namespace lab
         dbuf<int32_t> counts, ovf_rows, ovf2_rows, rp;
         dbuf<int>     novf_d;
         LAB_TRY(counts.alloc((size_t)m + 1, s));
-        LAB_TRY(ovf_rows.alloc((size_t)std::max(gs.count(4), 1), s));
+        // rows that may overflow their table: those of the 1024-slot class, and with
+        // tables smaller than the product bound (sym < 2) those of every class
+        const int may_ovf = tune.sym >= 2 ? gs.count(4)
+                                          : gs.count(1) + gs.count(2) + gs.count(3) + gs.count(4);
+        LAB_TRY(ovf_rows.alloc((size_t)std::max(may_ovf, 1), s));
         LAB_TRY(novf_d.alloc(2, s));
         LAB_CUDA(cudaMemsetAsync(novf_d.get(), 0, 2 * sizeof(int), s));
         LAB_CUDA(cudaMemsetAsync(counts.get(), 0, sizeof(int32_t) * (m + 1), s));
@@ -983,18 +995,19 @@ namespace lab
             stream_fork f(s, m); // lane tier and hash classes side by side
             LAB_TRY((esc_run<exp_gemm, 0>(e, m, tl, counts.get(), nullptr, nullptr, f.next())));
             LAB_TRY(launch_hash_classes<0>(gs, Ar, Br, counts.get(), nullptr, nullptr, nullptr,
-                                           ovf_rows.get(), novf_d.get(), f));
+                                           ovf_rows.get(), novf_d.get(), tune, f));
         }
-        if(gs.count(4))
+        if(may_ovf)
         {
-            // rows that filled 3/4 of the 1024-slot table get 4096 slots; their number
-            // is read on the device (a launch over the list's capacity), so no host
-            // round trip.  Rows that fill that one too (rare) are found at the sync
-            // below and go to the global sort tier.
-            LAB_TRY(ovf2_rows.alloc((size_t)gs.count(4), s));
-            LAB_TRY((launch_hash_cls<0, 4096, 4>(Ar, Br, ovf_rows.get(), gs.count(4), counts.get(),
+            // rows over their table's limit get 4096 slots; their number is read on the
+            // device (a launch over the list's capacity), so no host round trip.  Rows
+            // that fill that one too (rare) are found at the sync below and go to the
+            // global sort tier.
+            LAB_TRY(ovf2_rows.alloc((size_t)may_ovf, s));
+            LAB_TRY((launch_hash_cls<0, 4096, 4>(Ar, Br, ovf_rows.get(), may_ovf, counts.get(),
                                                  nullptr, nullptr, nullptr, ovf2_rows.get(),
-                                                 novf_d.get() + 1, s, novf_d.get())));
+                                                 novf_d.get() + 1, 3 * 4096 / 4, s,
+                                                 novf_d.get())));
             LAB_CUDA(cudaMemcpyAsync(hp + 32, novf_d.get() + 1, sizeof(int), cudaMemcpyDeviceToHost,
                                      s));
         }
@@ -1047,7 +1060,7 @@ namespace lab
             st = esc_run<exp_gemm, 1>(e2, m, tl, nullptr, out->col_ind, out->val, f.next());
             if(st == LAB_OK)
                 st = launch_hash_classes<1>(gn, Ar, Br, nullptr, out->row_ptr, out->col_ind,
-                                            out->val, nullptr, nullptr, f);
+                                            out->val, nullptr, nullptr, tune, f);
         }
         if(st == LAB_OK && gn.count(7))
         {

@@ -172,3 +172,33 @@ def test_hierarchy_matches_reference(gpu, reference):
     assert H.levels == Hr.levels
     for l in range(H.levels + 1):
         assert csr_equal(H.A(l).to_numpy(), Hr.A(l))
+
+
+@pytest.mark.parametrize("order", ["ascending", "any", "repeated"])
+@pytest.mark.parametrize("width", [3, 7, 40])
+def test_spgemm_row_sizes(gpu, oracle, width, order):
+    """Rows at the edges of the table classes of both passes (tables of 64 to 4096
+    slots, filled whole or to 3/4), with every product a column of its own and with
+    several products per column, from B rows shorter and longer than a group of
+    lanes; B's rows in ascending order, in any, or with a column twice."""
+    rng = np.random.default_rng(width)
+    sizes = [1, 32, 33, 48, 49, 96, 97, 100, 128, 129, 192, 193, 256, 257, 384, 385, 512, 513,
+             768, 769, 1024, 1025, 1536, 1537, 3072, 3100]
+    arp, aci, brp, bci = [0], [], [0], []
+    for k in sizes:
+        for times in (1, 3):  # products per column
+            cols = np.concatenate([rng.permutation(k) for _ in range(times)]) * 2 + k % 5
+            for q in range(0, cols.size, width):
+                row = np.unique(cols[q:q + width])
+                if order != "ascending":
+                    row = rng.permutation(row)
+                if order == "repeated":
+                    row = np.append(row, row[0])
+                aci.append(len(brp) - 1)
+                bci += row.tolist()
+                brp.append(len(bci))
+            arp.append(len(aci))
+    A = (np.array(arp, np.int32), np.array(aci, np.int32), rng.uniform(-1, 1, len(aci)))
+    B = (np.array(brp, np.int32), np.array(bci, np.int32), rng.uniform(-1, 1, len(bci)))
+    C = gpu.CsrMatrix.from_arrays(*A, n=len(brp) - 1).spgemm(gpu.CsrMatrix.from_arrays(*B, n=6300))
+    assert csr_equal(C.to_numpy(), oracle.spgemm((*A, len(brp) - 1), (*B, 6300)))

@@ -36,6 +36,10 @@ namespace lab
         int32_t* gate    = nullptr; // per 32 rows: a place solved two levels earlier, or -1
         double*  x       = nullptr; // the solution in the order of rows[]
         int      longest = 0;       // entries of the longest row
+        // solved by one cluster of so many CTAs (0: by the whole grid), which reads
+        // head[t] = (row, ent_ptr[t], ent_ptr[t + 1], value position of the first entry)
+        int   cluster = 0;
+        int4* head    = nullptr;
     };
 
     struct tri_plan
@@ -57,7 +61,7 @@ namespace lab
             return;
         for(tri_sched* t : {&A->tri->lower, &A->tri->upper})
             for(void* p : {(void*)t->rows, (void*)t->ent_ptr, (void*)t->ent_col,
-                           (void*)t->ent_src, (void*)t->gate, (void*)t->x})
+                           (void*)t->ent_src, (void*)t->gate, (void*)t->x, (void*)t->head})
                 if(p)
                     cudaFree(p);
         if(A->tri->diag)
@@ -373,13 +377,14 @@ namespace lab
     // The entries the reference visits in row i, in its order: forward
     // (host_csrtrsv.cpp:36-64) the row up to the first column right of the diagonal,
     // backward (66-90) the row right to left without the columns left of it.
-    // FILL false: their number; true: their columns' places and value positions.
+    // FILL false: their number, with stats[0] the largest and stats[1] set if some row
+    // has others between them; true: their columns' places and value positions.
     template <bool LOWER, bool FILL>
     __global__ void k_tri_entries(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
                                   const int32_t* __restrict__ order,
                                   const int32_t* __restrict__ place, int m, int32_t* ent_ptr,
                                   int32_t* __restrict__ ent_col, int32_t* __restrict__ ent_src,
-                                  int* longest)
+                                  int* stats)
     {
         const int t = blockIdx.x * blockDim.x + threadIdx.x;
         if(t >= m)
@@ -387,6 +392,7 @@ namespace lab
         const int i = order[t], a = rp[i], e = rp[i + 1];
         int       n = FILL ? ent_ptr[t] : 0;
         const int n0 = n;
+        int       first = 0;
         for(int k = 0; k < e - a; k++)
         {
             const int j = LOWER ? a + k : e - 1 - k;
@@ -402,14 +408,29 @@ namespace lab
                 ent_col[n] = c == i ? kTriDiag : place[c];
                 ent_src[n] = j;
             }
+            if(n == n0)
+                first = k;
             n++;
+            if(!FILL && k - first != n - 1 - n0)
+                atomicOr(stats + 1, 1);
         }
         if(!FILL)
         {
             ent_ptr[t] = n - n0;
-            if(n - n0 > *(volatile int*)longest)
-                atomicMax(longest, n - n0);
+            if(n - n0 > *(volatile int*)stats)
+                atomicMax(stats, n - n0);
         }
+    }
+
+    __global__ void k_tri_head(const int32_t* __restrict__ order,
+                               const int32_t* __restrict__ ent_ptr,
+                               const int32_t* __restrict__ ent_src, int m, int4* __restrict__ head)
+    {
+        const int t = blockIdx.x * blockDim.x + threadIdx.x;
+        if(t >= m)
+            return;
+        const int a = ent_ptr[t], e = ent_ptr[t + 1];
+        head[t] = make_int4(order[t], a, e, a < e ? ent_src[a] : 0);
     }
 
     // For the chunk of 32 rows that starts at row t0: the dependency nearest in the
@@ -432,21 +453,23 @@ namespace lab
         gate[w] = g;
     }
 
+    static int tri_cluster(bool lower, const tri_sched& t, int m);
+
     static lab_status tri_layout(const lab_csr_impl* A, bool lower, tri_sched& t, cudaStream_t s)
     {
         const int      m = (int)A->m;
         const unsigned g = (unsigned)ceil_div(m, 256);
         dbuf<int32_t>  place;
-        dbuf<int>      longest;
+        dbuf<int>      stats;
         int64_t        n = 0;
         LAB_TRY(place.alloc((size_t)m, s));
-        LAB_TRY(longest.alloc(1, s));
-        LAB_CUDA(cudaMemsetAsync(longest.get(), 0, sizeof(int), s));
+        LAB_TRY(stats.alloc(2, s));
+        LAB_CUDA(cudaMemsetAsync(stats.get(), 0, 2 * sizeof(int), s));
         LAB_TRY(dalloc(&t.ent_ptr, (size_t)m + 1, s));
         LAB_LAUNCH(k_tri_place, g, 256, 0, s, (const int32_t*)t.rows, m, place.get());
         LAB_LAUNCH((lower ? k_tri_entries<true, false> : k_tri_entries<false, false>), g, 256, 0, s,
                    A->row_ptr, A->col_ind, (const int32_t*)t.rows, (const int32_t*)place.get(), m,
-                   t.ent_ptr, (int32_t*)nullptr, (int32_t*)nullptr, longest.get());
+                   t.ent_ptr, (int32_t*)nullptr, (int32_t*)nullptr, stats.get());
         LAB_TRY(counts_to_rowptr(t.ent_ptr, t.ent_ptr, m, &n, s));
         LAB_TRY(dalloc(&t.ent_col, (size_t)std::max<int64_t>(n, 1), s));
         LAB_TRY(dalloc(&t.ent_src, (size_t)std::max<int64_t>(n, 1), s));
@@ -454,10 +477,20 @@ namespace lab
         LAB_TRY(dalloc(&t.x, (size_t)m, s));
         LAB_LAUNCH((lower ? k_tri_entries<true, true> : k_tri_entries<false, true>), g, 256, 0, s,
                    A->row_ptr, A->col_ind, (const int32_t*)t.rows, (const int32_t*)place.get(), m,
-                   t.ent_ptr, t.ent_col, t.ent_src, longest.get());
+                   t.ent_ptr, t.ent_col, t.ent_src, stats.get());
         LAB_LAUNCH(k_tri_gate, (unsigned)ceil_div(ceil_div(m, 32), 256), 256, 0, s,
                    (const int32_t*)t.ent_ptr, (const int32_t*)t.ent_col, m, t.gate);
-        return copy_d2h_sync(&t.longest, longest.get(), sizeof(int), s);
+        int h[2];
+        LAB_TRY(copy_d2h_sync(h, stats.get(), sizeof(h), s));
+        t.longest = h[0];
+        t.cluster = h[1] ? 0 : tri_cluster(lower, t, m);
+        if(t.cluster)
+        {
+            LAB_TRY(dalloc(&t.head, (size_t)m, s));
+            LAB_LAUNCH(k_tri_head, g, 256, 0, s, (const int32_t*)t.rows, (const int32_t*)t.ent_ptr,
+                       (const int32_t*)t.ent_src, m, t.head);
+        }
+        return LAB_OK;
     }
 
     lab_status tri_analyse(lab_csr_impl* A, cudaStream_t s)
@@ -713,6 +746,302 @@ namespace lab
         return (int)std::max<int64_t>(1, std::min<int64_t>(num_sms(), ceil_div(m, kTriBlock)));
     }
 
+    // ------------------------------------------------------------ one-cluster solve
+    // The same solve with x, in level order, in the shared memory of one cluster: a
+    // poll is a read of (distributed) shared memory instead of an L2 round trip, x needs
+    // no pass of its own to be marked pending, and chunks need no counter.  Chunk w of 32
+    // rows is CTA w % C's, and there warp (w / C) % kTriClWarps's, which takes its chunks
+    // in order: the first unsolved chunk's dependencies are solved and its warp has
+    // nothing before it, and a cluster's CTAs all run, so every wait ends.  The loads
+    // of a warp's next two chunks (heads, then entries) are in flight while it waits.
+    // Bound by the chain poll -> vote -> walk -> division -> store of each level.
+    // ILU(0)-PCG, against the grid: 64^3 (16 CTAs) 28.9 -> 20.4 ms, 20^3 (4) 3.7 -> 2.8
+    // ms, 100^2 (1) 29.4 -> 17.8 ms.  8 warps a CTA: 64^3 20.4 ms, 16: 20.8, 24: 24.5
+    // (waiting warps take issue slots from the ones that solve); waiting for a whole
+    // chunk to become ready before walking it (two more votes a round): 20.9 ms and
+    // 100^2 20.5 ms.
+    constexpr int kTriClBlock = 256;
+    constexpr int kTriClWarps = kTriClBlock / 32;
+    constexpr int kTriClMax   = 16;         // CTAs (16 needs the non-portable attribute)
+    constexpr int kTriClSmem  = 220 * 1024; // of x per CTA
+
+    template <bool ONE> // one CTA: its own shared memory
+    __device__ __forceinline__ uint64_t ld_cluster(uint32_t a)
+    {
+        uint64_t v;
+        if(ONE)
+            asm volatile("ld.relaxed.cta.shared::cta.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+        else
+            asm volatile("ld.relaxed.cluster.shared::cluster.b64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void cluster_barrier()
+    {
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+    }
+
+    template <bool LOWER, int PF, bool ONE>
+    __global__ void __launch_bounds__(kTriClBlock)
+        k_trsv_cluster(const int4* __restrict__ head, const int32_t* __restrict__ ent_col,
+                       const int32_t* __restrict__ gate, const double* __restrict__ v, int m,
+                       int unit, double dscale, const double* b, double* x, int logc, int32_t* ctl,
+                       const int* skip, unsigned idle_limit, int held)
+    {
+        if(skip && *skip)
+            return;
+        extern __shared__ __align__(16) uint64_t xs[];
+        const int      C = 1 << logc, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+        const int      chunks = (m + 31) >> 5;
+        const int      step   = kTriClWarps << logc;
+        const uint32_t xbase  = (uint32_t)__cvta_generic_to_shared(xs);
+        uint32_t       rank;
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+        for(int q = threadIdx.x; q < ((chunks + C - 1) >> logc) * 32; q += kTriClBlock)
+            xs[q] = kTriPending;
+        cluster_barrier();
+        auto where = [&](int p) { // shared address of place p
+            uint32_t  a = xbase + ((((uint32_t)p >> 5) >> logc) * 32 + (p & 31)) * 8;
+            uint32_t  r;
+            if(ONE)
+                return a;
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"((p >> 5) & (C - 1)));
+            return r;
+        };
+        struct held_row
+        {
+            int      i = -1, k = 0, e = 0, src = 0, pc[PF];
+            double   pv[PF], b = 0.0;
+        };
+        auto get_head = [&](int w) {
+            const int t = w * 32 + lane;
+            return (w < chunks && t < m) ? head[t] : make_int4(-1, 0, 0, 0);
+        };
+        auto hold = [&](held_row& r) { // entries k .. k + PF
+#pragma unroll
+            for(int q = 0; q < PF; q++)
+            {
+                const bool ok = r.k + q < r.e;
+                r.pc[q]       = ok ? ent_col[r.k + q] : kTriDiag;
+                r.pv[q]       = ok ? v[LOWER ? r.src + q : r.src - q] : 0.0;
+            }
+        };
+        auto get_row = [&](const int4& h) {
+            held_row r;
+            r.i   = h.x;
+            r.k   = h.y;
+            r.e   = h.z;
+            r.src = h.w;
+            hold(r);
+            r.b = h.x >= 0 ? b[h.x] : 0.0;
+            return r;
+        };
+        int      w = (int)rank + (wid << logc);
+        held_row row  = get_row(get_head(w));
+        int4     next = get_head(w + step);
+        int      g    = w < chunks ? gate[w] : -1;
+        bool     ok   = true; // false: a wait ran out
+        while(w < chunks && ok)
+        {
+            const int4     next2 = get_head(w + 2 * step);
+            const held_row rown  = get_row(next);
+            const int      gn    = w + step < chunks ? gate[w + step] : -1;
+
+            bool     done = row.i < 0;
+            double   acc = LOWER ? 0.0 : row.b, d = 1.0;
+            uint32_t at[PF];
+            uint64_t xv[PF];
+            unsigned need = 0, idle = 0;
+            auto     wants = [&]() {
+                need = 0;
+#pragma unroll
+                for(int q = 0; q < PF; q++)
+                {
+                    at[q] = row.pc[q] >= 0 ? where(row.pc[q]) : 0;
+                    need |= (unsigned)(row.pc[q] >= 0) << q;
+                    xv[q] = 0;
+                }
+            };
+            // a round without progress; false: the wait ran out
+            auto wait = [&]() {
+                const bool out = ++idle >= idle_limit;
+                if(out && lane == 0)
+                    atomicExch(ctl + 1, 1);
+                return !(out || ((idle & 1023u) == 0 &&
+                                 __any_sync(0xffffffffu, ld_acquire(ctl + 1) != 0)));
+            };
+            wants();
+            if(g >= 0)
+            {
+                const uint32_t ga = where(g);
+                while(ok && __any_sync(0xffffffffu, ld_cluster<ONE>(ga) == kTriPending))
+                {
+                    ok = wait();
+                    __nanosleep(32);
+                }
+                idle = 0;
+            }
+            while(ok)
+            {
+                uint64_t u[PF];
+#pragma unroll
+                for(int q = 0; q < PF; q++)
+                    u[q] = (need >> q & 1u) ? ld_cluster<ONE>(at[q]) : kTriPending;
+#pragma unroll
+                for(int q = 0; q < PF; q++)
+                    if(u[q] != kTriPending)
+                    {
+                        xv[q] = u[q];
+                        need &= ~(1u << q);
+                    }
+                const bool ready = !done && need == 0;
+                if(!__any_sync(0xffffffffu, ready))
+                {
+                    ok = wait();
+                    continue;
+                }
+                idle = 0;
+                if(ready)
+                {
+                    bool stop = false;
+#pragma unroll
+                    for(int q = 0; q < PF; q++)
+                    {
+                        if(stop || row.k + q >= row.e)
+                            continue;
+                        if(row.pc[q] >= 0)
+                        {
+                            const double xc = __longlong_as_double((long long)xv[q]);
+                            acc = LOWER ? fma(row.pv[q], xc, acc)
+                                        : __dsub_rn(acc, __dmul_rn(row.pv[q], xc));
+                        }
+                        else if(!unit)
+                            d = (LOWER && dscale != 0.0) ? __dmul_rn(row.pv[q], dscale) : row.pv[q];
+                        else
+                            stop = LOWER;
+                    }
+                    row.k += PF;
+                    if(!stop && row.k < row.e)
+                    {
+                        row.src += LOWER ? PF : -PF;
+                        hold(row);
+                        wants();
+                    }
+                    else
+                    {
+                        done = true;
+                        need = 0;
+                        if(row.i != held) // else its value stays pending
+                        {
+                            double r = LOWER ? __dsub_rn(row.b, acc) : acc;
+                            if(!LOWER || !unit)
+                                r = __ddiv_rn(r, d);
+                            asm volatile("st.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(
+                                             xbase + ((w >> logc) * 32 + lane) * 8),
+                                         "l"(__double_as_longlong(r))
+                                         : "memory");
+                            x[row.i] = r;
+                        }
+                    }
+                }
+                if(__all_sync(0xffffffffu, done))
+                    break;
+            }
+            row  = rown;
+            next = next2;
+            g    = gn;
+            w += step;
+        }
+        __syncwarp();
+        cluster_barrier(); // no CTA leaves while others may read its shared memory
+    }
+
+    template <bool LOWER, int PF, bool ONE>
+    static lab_status trsv_cluster_launch(const lab_csr_impl* A, const tri_plan* p,
+                                          const tri_sched& t, int C, bool unit, double dscale,
+                                          const double* b, double* x, cudaStream_t s,
+                                          const int* skip, int m, int* active)
+    {
+        static const cudaError_t attr = [] {
+            cudaError_t e = cudaFuncSetAttribute(k_trsv_cluster<LOWER, PF, ONE>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 kTriClSmem);
+            return e != cudaSuccess
+                       ? e
+                       : cudaFuncSetAttribute(k_trsv_cluster<LOWER, PF, ONE>,
+                                              cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        }();
+        LAB_CUDA(attr);
+        const int           chunks = (int)ceil_div(m, 32);
+        cudaLaunchConfig_t  cfg{};
+        cudaLaunchAttribute at{};
+        at.id               = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = (unsigned)C;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.gridDim          = dim3((unsigned)C);
+        cfg.blockDim         = dim3(kTriClBlock);
+        cfg.dynamicSmemBytes = sizeof(double) * 32 * (size_t)ceil_div(chunks, C);
+        cfg.stream           = s;
+        cfg.attrs            = &at;
+        cfg.numAttrs         = 1;
+        if(active)
+        {
+            LAB_CUDA(cudaOccupancyMaxActiveClusters(active, k_trsv_cluster<LOWER, PF, ONE>, &cfg));
+            return LAB_OK;
+        }
+        int logc = 0;
+        while((1 << logc) < C)
+            logc++;
+        LAB_CUDA(cudaLaunchKernelEx(&cfg, k_trsv_cluster<LOWER, PF, ONE>, (const int4*)t.head,
+                                    (const int32_t*)t.ent_col, (const int32_t*)t.gate,
+                                    (const double*)A->val, m, (int)unit, dscale, b, x, logc, p->ctl,
+                                    skip, p->idle_limit ? p->idle_limit : kTriIdle, p->held_row));
+        g_launches.fetch_add(1);
+        return LAB_OK;
+    }
+
+    static lab_status trsv_cluster(bool lower, const lab_csr_impl* A, const tri_plan* p,
+                                   const tri_sched& t, int C, bool unit, double dscale,
+                                   const double* b, double* x, cudaStream_t s, const int* skip,
+                                   int m, int* active)
+    {
+        const auto launch
+            = C == 1 ? (lower ? (t.longest <= 4 ? trsv_cluster_launch<true, 4, true>
+                                                : trsv_cluster_launch<true, 8, true>)
+                              : (t.longest <= 4 ? trsv_cluster_launch<false, 4, true>
+                                                : trsv_cluster_launch<false, 8, true>))
+                     : (lower ? (t.longest <= 4 ? trsv_cluster_launch<true, 4, false>
+                                                : trsv_cluster_launch<true, 8, false>)
+                              : (t.longest <= 4 ? trsv_cluster_launch<false, 4, false>
+                                                : trsv_cluster_launch<false, 8, false>));
+        return launch(A, p, t, C, unit, lower ? dscale : 0.0, b, x, s, skip, m, active);
+    }
+
+    // CTAs of the cluster that solves this triangle, 0: the grid does.
+    //  - A mean level of 64 rows (two chunks) a CTA: fewer CTAs poll closer memory, more
+    //    solve a level's chunks side by side (40^3, 542 rows a level: 16 CTAs 8.3 ms, 8
+    //    8.6, 4 10.3; 100^2, 50 rows: 1 CTA 17.8 ms, 2 20.8), and as many as x needs.
+    //  - Up to 4096 rows a level: 16 SMs hold 4096 rows in flight, a level of more than
+    //    that costs them several round trips to L2 where 148 SMs need one.
+    static int tri_cluster(bool lower, const tri_sched& t, int m)
+    {
+        const int levels = std::max(1, (int)t.ptr.size() - 1);
+        const int chunks = (int)ceil_div(m, 32);
+        const int width  = (int)ceil_div(m, levels);
+        if(width > 4096)
+            return 0;
+        int C = 1;
+        while(C < kTriClMax && (C * 64 < width ||
+                                (int64_t)ceil_div(chunks, C) * 256 > kTriClSmem))
+            C *= 2;
+        if((int64_t)ceil_div(chunks, C) * 256 > kTriClSmem)
+            return 0;
+        int active = 0;
+        if(trsv_cluster(lower, nullptr, nullptr, t, C, false, 0.0, nullptr, nullptr, nullptr,
+                        nullptr, m, &active) != LAB_OK)
+            cudaGetLastError();
+        return active > 0 ? C : 0;
+    }
+
     template <bool LOWER, int PF>
     static lab_status trsv_launch(const lab_csr_impl* A, const tri_plan& p, const tri_sched& t,
                                   bool unit, double dscale, const double* b, double* x,
@@ -742,6 +1071,8 @@ namespace lab
             LAB_CUDA(cudaMemcpyAsync(p.scratch, b, sizeof(double) * m, cudaMemcpyDeviceToDevice, s));
             b = p.scratch;
         }
+        if(t.cluster)
+            return trsv_cluster(lower, A, &p, t, t.cluster, unit, dscale, b, x, s, skip, m, nullptr);
         LAB_LAUNCH(k_trsv_prep, (unsigned)std::min<int64_t>(ceil_div(m, 256), 4 * num_sms()), 256,
                    0, s, t.x, m, p.ctl, skip);
         // 4 held entries cover a triangle of a 5- or 7-point operator with its diagonal

@@ -289,3 +289,35 @@ def test_trsv_row_lengths_bit_exact(gpu, oracle, n, k, shuffle):
             L.call("lab_csrtrsv", dA.h, int(lower), int(unit), gpu.ptr(y), gpu.ptr(y),
                    gpu.stream_handle())
             assert np.array_equal(_bits(y.cpu().numpy()), want)
+
+
+def _two_levels(n):
+    """Half the rows depend on one of the other half: two levels of n / 2 rows."""
+    h = n // 2
+    rng = np.random.default_rng(n)
+    lo, hi = rng.permutation(h), h + rng.permutation(h)
+    rp = np.arange(0, 2 * n + 1, 2)
+    ci = np.empty((n, 2), np.int64)
+    ci[:h] = np.stack([np.arange(h), hi], 1)
+    ci[h:] = np.stack([lo, np.arange(h, n)], 1)
+    v = np.where(ci == np.arange(n)[:, None], 3.0, rng.uniform(-1, 1, (n, 2)))
+    return rp.astype(np.int32), ci.reshape(-1).astype(np.int32), v.reshape(-1)
+
+
+@pytest.mark.parametrize("make", [
+    lambda: P.poisson2d(130),       # levels of 65 rows: clusters of 2 CTAs
+    lambda: P.poisson3d(20),        # 138: 4
+    lambda: P.poisson3d(30),        # 307: 8
+    lambda: P.poisson3d(41),        # 570: 16
+    lambda: P.poisson2d(700),       # more than 16 CTAs' shared memory holds: the grid
+    lambda: _two_levels(9000),      # wide and shallow: the grid
+], ids=["c2", "c4", "c8", "c16", "large", "wide"])
+def test_trsv_cluster_sizes_bit_exact(gpu, oracle, make):
+    A = make()[:3]
+    b = np.random.default_rng(5).uniform(-1, 1, A[0].size - 1)
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    for lower in (True, False):
+        want = _bits(oracle.trsv(A, b, lower, False))
+        for _ in range(2):
+            x = dA.trsv(gpu.vec(b), lower=lower, unit_diag=False)
+            assert np.array_equal(_bits(x.cpu().numpy()), want)

@@ -1213,7 +1213,17 @@ namespace lab
     // (K, nseg) grid: K CTAs per segment, each over a fixed contiguous chunk, the
     // last CTA of a segment (per-segment ticket) reducing the K partials in order
     // -- deterministic, and a converged segment is skipped (convergence mask).
-    constexpr int kSegK = 8;
+    // CTAs a segment in its reductions and vector updates: eight, and with few segments
+    // as many as give every SM eight CTAs in all, of 512 rows or more.  4 systems of up
+    // to 256^2 rows: 2.43 ms a solve with 8, 2.16 with 64; 256 of them: 17.3 ms with 8
+    // or 16, 17.8 with 32; 150 of up to 60^2: 1.97 ms with 8, 2.23 with 16.
+    constexpr int kSegMax = 64;
+    static int    seg_ctas(int nseg, int64_t rows)
+    {
+        const int     n = std::max(nseg, 1);
+        const int64_t k = std::min<int64_t>(ceil_div(8 * num_sms(), n), rows / n / 512);
+        return (int)std::min<int64_t>(kSegMax, std::max<int64_t>(8, k));
+    }
     // global flags: [0] = all done, [1] = active segments, [2] = max_iter,
     // [3] = passes of the device-side iteration loop
     struct seg_ws
@@ -1225,7 +1235,7 @@ namespace lab
         double*       sc      = nullptr; // [nseg][G_N]
         int*          sf      = nullptr; // [nseg][GF_N]
         int*          gflags  = nullptr; // [4]
-        double*       partial = nullptr; // [4 slots][nseg][kSegK]
+        double*       partial = nullptr; // [4 slots][nseg][ctas]
         unsigned int* tickets = nullptr; // [4 slots][nseg]
         double        rtol = 0, atol = 0;
         void release()
@@ -1241,7 +1251,7 @@ namespace lab
                                               int64_t& b)
     {
         const int64_t s0 = off[s], s1 = off[s + 1];
-        const int64_t ch = (s1 - s0 + kSegK - 1) / kSegK;
+        const int64_t ch = (s1 - s0 + gridDim.x - 1) / gridDim.x;
         a                = s0 + k * ch;
         b                = min(s1, a + ch);
     }
@@ -1254,10 +1264,20 @@ namespace lab
         if(threadIdx.x == 0)
         {
             __threadfence();
-            last = atomicAdd(t, 1u) == kSegK - 1;
+            last = atomicAdd(t, 1u) == gridDim.x - 1;
         }
         __syncthreads();
         return last;
+    }
+
+    // The CTAs' partial results of segment s, in shared memory (every thread of its last CTA).
+    __device__ __forceinline__ const double* seg_partials(const double* partial, int s)
+    {
+        __shared__ double all[kSegMax];
+        if(threadIdx.x < gridDim.x)
+            all[threadIdx.x] = __ldcg(partial + (size_t)s * gridDim.x + threadIdx.x);
+        __syncthreads();
+        return all;
     }
 
     // (x, y) per segment -> sc[s][slot]; OP 1: max |x|
@@ -1273,22 +1293,21 @@ namespace lab
         int64_t a, b;
         seg_range(off, s, k, a, b);
         double acc = 0.0;
+#pragma unroll 4
         for(int64_t i = a + threadIdx.x; i < b; i += 256)
             acc = OP == 0 ? acc + x[i] * y[i] : nanmax(acc, fabs(x[i]));
         double bs = OP == 0 ? block_sum<256>(acc) : block_max<256>(acc);
         if(threadIdx.x == 0)
-            partial[(size_t)s * kSegK + k] = bs;
+            partial[(size_t)s * gridDim.x + k] = bs;
         (void)nseg;
         if(seg_ticket(&tickets[s]))
         {
+            const double* all = seg_partials(partial, s);
             if(threadIdx.x == 0)
             {
                 double t = 0.0;
-                for(int j = 0; j < kSegK; j++)
-                {
-                    double v = __ldcg(partial + (size_t)s * kSegK + j);
-                    t        = OP == 0 ? t + v : nanmax(t, v);
-                }
+                for(int j = 0; j < (int)gridDim.x; j++)
+                    t = OP == 0 ? t + all[j] : nanmax(t, all[j]);
                 sc[s * G_N + slot] = t;
                 tickets[s]         = 0;
             }
@@ -1319,6 +1338,7 @@ namespace lab
         int64_t      a, b;
         seg_range(off, s, k, a, b);
         double acc = 0.0;
+#pragma unroll 4
         for(int64_t i = a + threadIdx.x; i < b; i += 256)
         {
             x[i]      = alpha == 1.0 ? __dadd_rn(p[i], x[i]) : __dadd_rn(__dmul_rn(alpha, p[i]), x[i]);
@@ -1328,14 +1348,15 @@ namespace lab
         }
         double bs = block_max<256>(acc);
         if(threadIdx.x == 0)
-            partial[(size_t)s * kSegK + k] = bs;
+            partial[(size_t)s * gridDim.x + k] = bs;
         if(seg_ticket(&tickets[s]))
         {
+            const double* all = seg_partials(partial, s);
             if(threadIdx.x == 0)
             {
                 double t = 0.0;
-                for(int j = 0; j < kSegK; j++)
-                    t = nanmax(t, __ldcg(partial + (size_t)s * kSegK + j));
+                for(int j = 0; j < (int)gridDim.x; j++)
+                    t = nanmax(t, all[j]);
                 tickets[s]          = 0;
                 sc[s * G_N + G_RN]  = t;
                 double r0           = sc[s * G_N + G_R0];
@@ -1359,6 +1380,7 @@ namespace lab
         const double beta = sc[s * G_N + G_GNEW] / sc[s * G_N + G_GAMMA];
         int64_t      a, b;
         seg_range(off, s, k, a, b);
+#pragma unroll 4
         for(int64_t i = a + threadIdx.x; i < b; i += 256)
             p[i] = beta == 0.0 ? z[i] : __dadd_rn(z[i], __dmul_rn(beta, p[i]));
         if(seg_ticket(&tickets[s]))
@@ -1454,7 +1476,7 @@ namespace lab
         al(&w.sc, (size_t)nseg * G_N);
         al(&w.sf, (size_t)nseg * GF_N);
         al(&w.gflags, 4);
-        al(&w.partial, (size_t)4 * nseg * kSegK);
+        al(&w.partial, (size_t)4 * nseg * seg_ctas(nseg, w.total));
         al(&w.tickets, (size_t)4 * nseg);
         if(st != LAB_OK)
         {
@@ -1465,9 +1487,9 @@ namespace lab
         cudaMemsetAsync(w.tickets, 0, sizeof(unsigned int) * 4 * nseg, s);
         cudaMemsetAsync(w.gflags, 0, sizeof(int) * 4, s);
         cudaMemsetAsync(w.sf, 0, sizeof(int) * nseg * GF_N, s);
-        const dim3 grid(kSegK, nseg);
+        const dim3 grid(seg_ctas(nseg, w.total), nseg);
         const int* skip = w.gflags;
-        auto       red  = [&](int slotbuf) { return w.partial + (size_t)slotbuf * nseg * kSegK; };
+        auto       red  = [&](int slotbuf) { return w.partial + (size_t)slotbuf * nseg * grid.x; };
         auto       tik  = [&](int slotbuf) { return w.tickets + (size_t)slotbuf * nseg; };
 
         cudaEvent_t t0, t1;

@@ -1020,8 +1020,9 @@ namespace lab
     //  - A mean level of 64 rows (two chunks) a CTA: fewer CTAs poll closer memory, more
     //    solve a level's chunks side by side (40^3, 542 rows a level: 16 CTAs 8.3 ms, 8
     //    8.6, 4 10.3; 100^2, 50 rows: 1 CTA 17.8 ms, 2 20.8), and as many as x needs.
-    //  - Up to 4096 rows a level: 16 SMs hold 4096 rows in flight, a level of more than
-    //    that costs them several round trips to L2 where 148 SMs need one.
+    //  - Up to 4096 rows a level: 16 SMs hold 4096 rows in flight, and a lower solve
+    //    with levels of 500 / 1500 / 3000 / 4096 / 4200 rows takes 277 / 165 / 116 / 90 us
+    //    here against 384 / 216 / 136 / 95 on the grid, which is level with it beyond.
     static int tri_cluster(bool lower, const tri_sched& t, int m)
     {
         const int levels = std::max(1, (int)t.ptr.size() - 1);

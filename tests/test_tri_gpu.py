@@ -321,3 +321,18 @@ def test_trsv_cluster_sizes_bit_exact(gpu, oracle, make):
         for _ in range(2):
             x = dA.trsv(gpu.vec(b), lower=lower, unit_diag=False)
             assert np.array_equal(_bits(x.cpu().numpy()), want)
+
+
+def test_trsv_bounded_wait_on_grid(gpu, oracle):
+    """The bounded wait of the form that solves on the whole grid (a wide triangle)."""
+    from linalglib_b200 import _lib as L
+    A = _two_levels(9000)
+    b = np.random.default_rng(6).uniform(-1, 1, 9000)
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    L.call("lab_csrtrsv_wait_control", dA.h, 1 << 12, 0, gpu.stream_handle())
+    bx, x = gpu.vec(b), gpu.vec(np.zeros(9000))
+    st = L.lib().lab_csrtrsv(dA.h, 1, 0, gpu.ptr(bx), gpu.ptr(x), gpu.stream_handle())
+    assert st == L.LAB_TIMEOUT, L.lib().lab_last_error().decode()
+    L.call("lab_csrtrsv_wait_control", dA.h, 0, -1, gpu.stream_handle())
+    x = dA.trsv(gpu.vec(b), lower=True)
+    assert np.array_equal(_bits(x.cpu().numpy()), _bits(oracle.trsv(A, b, True, False)))

@@ -9,7 +9,8 @@
 // order, reading a dependency once its value is no longer marked pending.  A
 // chunk only waits on rows claimed before it, by warps that are running, so
 // every wait ends; the waits are still bounded (an error flag is set and the
-// kernel returns).  The factorizations run one launch per level.
+// kernel returns).  Triangles that fit do the same inside one cluster, with x in its
+// shared memory.  The factorizations run one launch per level.
 // Every row is computed by one thread in exactly the reference's operation
 // order (host_csrtrsv.cpp, host_csrilu0.cpp, host_csric0.cpp), so the results
 // are bit-identical to the reference's sequential loops.

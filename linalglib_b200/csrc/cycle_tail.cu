@@ -103,7 +103,11 @@ namespace lab
 
     // The rows of one pass.  A pass is a chain of shared-memory latencies, so what
     // does not depend on one another is loaded together and without branches
-    // (entries beyond the row's end at a clamped position, the sum unchanged).
+    // (positions outside the row at a clamped one inside it, the sum unchanged).  A
+    // row without entries, and a lane past the last row, has no position inside it
+    // and loads none: its loop starts at its end (the quad below starts before
+    // the row, so it would be entered, and what lies past the operator's last entry
+    // is no column).
     template <class T, class IT>
     __device__ __forceinline__ void tail_rows(const int4 q0, const int4 q1, const int4 q2,
                                               const int4 q3, unsigned char* sm, T om, T* dst)
@@ -130,7 +134,8 @@ namespace lab
             const T   pd = reinterpret_cast<const T*>(sm + q3.x)[r];
             T         s  = T(0);
 #pragma unroll 1
-            for(int j = quad ? (a0 & ~3) + 4 * lane : a0 + lane; j < a1; j += U * W)
+            for(int j = a0 == a1 ? a1 : quad ? (a0 & ~3) + 4 * lane : a0 + lane; j < a1;
+                j += U * W)
             {
                 T vv[U], xv[U];
 #pragma unroll

@@ -39,3 +39,38 @@ def test_tail_matches_oracle_cycle(gpu, oracle, name, make, n1, n2):
             z = z.cpu().numpy()
             assert np.max(np.abs(z[shift:shift + m] - zo)) <= tol * np.max(np.abs(zo))
             assert np.all(z[:shift] == 7.0) and np.all(z[shift + m:] == 7.0)
+
+
+def _lone(A, rows):
+    """A with the rows and columns of the given unknowns cut down to their diagonal: they
+    have no strong neighbour, so no aggregate, and their rows of P are empty."""
+    rp, ci, v = A[:3]
+    r = np.repeat(np.arange(rp.size - 1), np.diff(rp))
+    keep = ~(np.isin(r, rows) | np.isin(ci, rows)) | (r == ci)
+    cnt = np.bincount(r[keep], minlength=rp.size - 1)
+    return np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32), ci[keep], v[keep]
+
+
+@pytest.mark.parametrize("lanes", [0, 2, 8, 32])
+@pytest.mark.parametrize("make", [lambda: P.poisson2d(14), lambda: P.poisson2d(16),
+                                  lambda: P.poisson3d(13)], ids=["2d 14", "2d 16", "3d 13"])
+def test_tail_empty_rows(gpu, oracle, make, lanes):
+    """Empty rows of P, in the middle and at the end (its entries not a multiple of four,
+    so that the row starts inside a group of four), with P and R summed by several
+    lanes a row: a row without entries reads none."""
+    A = make()
+    m = A[0].size - 1
+    A = _lone(A, [m // 2, m - 2, m - 1])
+    H = gpu.Hierarchy(gpu.CsrMatrix.from_arrays(*A), kind=L.AMG_SA)
+    rp = H.P(0).to_numpy()[0]
+    assert rp[m - 2] == rp[m] and rp[m // 2] == rp[m // 2 + 1]
+    r = np.random.default_rng(m).uniform(-1, 1, m)
+    zo = oracle.amg_setup(A, kind=0).vcycle(r, n1=1, n2=1, omega=2.0 / 3.0, coarse=1)
+    if lanes:
+        for l in range(H.levels):
+            for M in (H.P(l), H.R(l)):
+                M.set_algorithm(L.SPMV_VECTOR, lanes)
+    for precision, tol in ((L.PREC_FP64, 1e-12), (L.PREC_FP32, 4e-5)):
+        M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0, precision=precision))
+        z = M.apply(gpu.vec(r)).cpu().numpy()
+        assert np.max(np.abs(z - zo)) <= tol * np.max(np.abs(zo))

@@ -479,12 +479,16 @@ namespace lab
     // Levels l+1 .. L form a fused tail when the cycle is a V-cycle with Jacobi
     // smoothing (n1 >= 1) from a zero guess, level l's operators are not BF16, every
     // operator below l + 1 fits shared memory with the level vectors, and the
-    // coarsest level is solved by a 1x1 division or the dense inverse.  One CTA stays
+    // coarsest level is solved by a 1x1 division or a dense inverse of up to kTailInv
+    // rows (every pass of the cycle in its own launch against the tail, us a cycle: 64
+    // rows 10.7 / 9.1, 74 23.3 / 21.9, 82 11.9 / 11.3, 83 23.5 / 24.0, 98 11.6 / 13.1,
+    // 170 12.6 / 17.0: one CTA reads all of the inverse).  One CTA stays
     // ahead of the 3 to 4 us that a separate launch costs up to about 16 entries per
     // thread and pass (kTailEntries).  R and P of level l join the launch up to
     // kTailEdge entries: above that one SM's share of the memory bandwidth costs more
     // than the two launches (9,433 entries: 25 us against 6).
     constexpr int64_t kTailEntries = 16 * kTailNT;
+    constexpr int64_t kTailInv     = 80;
 
     int tail_ok(const hierarchy_impl* h, const lab_amg_options* o, int l)
     {
@@ -493,7 +497,7 @@ namespace lab
            l >= L || nl > kTailMax || level_bf16(o, l) || !device_status_word())
             return TAIL_NONE;
         const int64_t nc = h->A[L]->m;
-        if(nc != 1 && !(nc > 1 && nc <= 1024 && o->coarse == LAB_COARSE_DIRECT && h->coarse_inv))
+        if(nc != 1 && !(nc > 1 && nc <= kTailInv && o->coarse == LAB_COARSE_DIRECT && h->coarse_inv))
             return TAIL_NONE;
         if(2 + (int64_t)(nl - 1) * (2 + (int64_t)o->n1 + std::max(o->n2, 0)) + 1 > kTailPasses)
             return TAIL_NONE;

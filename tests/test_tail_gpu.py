@@ -74,3 +74,20 @@ def test_tail_empty_rows(gpu, oracle, make, lanes):
         M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0, precision=precision))
         z = M.apply(gpu.vec(r)).cpu().numpy()
         assert np.max(np.abs(z - zo)) <= tol * np.max(np.abs(zo))
+
+
+@pytest.mark.parametrize("n, launches", [(14, 3), (16, 3), (18, 5), (20, 5), (26, 5)])
+def test_tail_dense_coarse_rows(gpu, oracle, n, launches):
+    """Coarsest levels of 50 and 64 rows are solved in the tail's one launch (after the
+    first pass over level 0 and before its last), of 82, 98 and 170 rows on the whole GPU."""
+    A = P.poisson2d(n)
+    H = gpu.Hierarchy(gpu.CsrMatrix.from_arrays(*A), kind=L.AMG_SA, max_level=1)
+    M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0))
+    r = np.random.default_rng(n).uniform(-1, 1, n * n)
+    rd = gpu.vec(r)
+    n0 = gpu.launch_count()
+    z = M.apply(rd)
+    assert gpu.launch_count() - n0 == launches
+    zo = oracle.amg_setup(A, kind=0, max_level=1).vcycle(r, n1=1, n2=1, omega=2.0 / 3.0, coarse=1)
+    # the two inverses round differently, by the coarsest operator's condition number (< 1e4)
+    assert np.max(np.abs(z.cpu().numpy() - zo)) <= 1e-11 * np.max(np.abs(zo))

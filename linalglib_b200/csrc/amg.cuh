@@ -42,6 +42,7 @@ namespace lab
         double* coarse_inv   = nullptr;
         float*  coarse_inv32 = nullptr;
         int     coarse_n     = 0;
+        int*    status       = nullptr; // device word counting waits that ran out (borrowed)
         int     coarse_singular = 0;
     };
 

@@ -896,6 +896,8 @@ namespace lab
                 LAB_TRY(build_colouring(A, w, s));
         }
         LAB_TRY(build_coarse(h, o->coarse, s));
+        // the first call allocates, which a cycle inside a caller's capture must not
+        h->status   = device_status_word();
         h->ws_ready = 1;
         return LAB_OK;
     }

@@ -494,7 +494,7 @@ namespace lab
     {
         const int L = h->levels, nl = L - l;
         if(o->cycle != LAB_CYCLE_V || o->smoother != LAB_SMOOTH_JACOBI || o->n1 < 1 ||
-           l >= L || nl > kTailMax || level_bf16(o, l) || !device_status_word())
+           l >= L || nl > kTailMax || level_bf16(o, l) || !h->status)
             return TAIL_NONE;
         const int64_t nc = h->A[L]->m;
         if(nc != 1 && !(nc > 1 && nc <= kTailInv && o->coarse == LAB_COARSE_DIRECT && h->coarse_inv))
@@ -536,7 +536,7 @@ namespace lab
         tail_plan<T> t;
         t.build(h, c.o, l, edge, wr, cur, dst);
         t.a.skip   = c.skip;
-        t.a.status = device_status_word();
+        t.a.status = h->status;
         static const cudaError_t attr = cudaFuncSetAttribute(
             k_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem);
         LAB_CUDA(attr);

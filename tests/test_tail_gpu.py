@@ -91,3 +91,31 @@ def test_tail_dense_coarse_rows(gpu, oracle, n, launches):
     zo = oracle.amg_setup(A, kind=0, max_level=1).vcycle(r, n1=1, n2=1, omega=2.0 / 3.0, coarse=1)
     # the two inverses round differently, by the coarsest operator's condition number (< 1e4)
     assert np.max(np.abs(z.cpu().numpy() - zo)) <= 1e-11 * np.max(np.abs(zo))
+
+
+def test_first_cycle_of_a_process_can_be_captured(gpu):
+    """A preconditioner's first application may run inside the caller's stream capture:
+    what the cycle needs is allocated when the preconditioner is built.  (In a process
+    of its own, where nothing has run before.)"""
+    import os
+    import subprocess
+    import sys
+    code = """
+import numpy as np, torch
+from linalglib_b200 import core, _lib as L, problems as P
+A = P.poisson2d(61)
+r = core.vec(np.random.default_rng(0).uniform(-1, 1, 61 * 61))
+for precision in (L.PREC_FP64, L.PREC_FP32):
+    M = core.Preconditioner.amg(core.Hierarchy(core.CsrMatrix.from_arrays(*A)),
+                                core.amg_options(omega=2.0 / 3.0, precision=precision))
+    z = torch.zeros_like(r)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        M.apply(r, z)
+    g.replay()
+    assert torch.equal(z, M.apply(r)) and float(z.abs().max()) > 0.0
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert p.returncode == 0, p.stderr[-2000:]

@@ -71,10 +71,13 @@ LAB_API lab_status lab_init(int device);
 LAB_API lab_status lab_synchronize(lab_stream s);
 /* Number of kernel launches issued by this library since load (all threads). */
 LAB_API int64_t lab_launch_count(void);
-/* How many bounded device-side waits of the streaming row kernels ran out on the
- * current device since the library was loaded (0 in normal operation: a wait
- * that runs out ends its kernel early instead of hanging the GPU, and the rows
- * it had not reached are left unwritten).  No reference counterpart. */
+/* How many bounded device-side waits of the streaming row kernels and of the V-cycle's
+ * fused last levels ran out on the current device since the library was loaded (0 in
+ * normal operation: a wait that runs out ends its kernel early instead of hanging the
+ * GPU).  A streaming row kernel leaves the rows it had not reached unwritten.  A cycle's
+ * result is NaN, so a solve with it ends at once and returns LAB_TIMEOUT; the calls
+ * that only enqueue (lab_precond_apply, lab_amg_cycle) return LAB_OK before it is known.
+ * No reference counterpart. */
 LAB_API lab_status lab_wait_timeouts(int64_t* count, lab_stream s);
 /* Allocate / free library device memory (stream ordered). */
 LAB_API lab_status lab_malloc(void** p, size_t bytes, lab_stream s);
@@ -342,6 +345,10 @@ LAB_API lab_status lab_hierarchy_level(lab_hierarchy h, int level, lab_csr* A, l
                                        lab_csr* R);
 /* Setup timing of the last lab_amg_setup on this hierarchy, milliseconds. */
 LAB_API lab_status lab_hierarchy_setup_ms(lab_hierarchy h, double* ms);
+/* The bound, in polls, of the waits in h's cycles (0: the default), and whether they wait
+ * for something that never comes (to test the bound).  Set before solving with h:
+ * iteration graphs captured earlier keep theirs. */
+LAB_API lab_status lab_hierarchy_wait_control(lab_hierarchy h, int64_t polls, int held);
 /* Write a built hierarchy (every A_l, P_l, R_l) to a binary file, and load one
  * back onto the device: a loaded hierarchy is bit-identical to the saved one, so
  * reruns on the same operator skip the setup.  No counterpart in the reference

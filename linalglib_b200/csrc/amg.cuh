@@ -43,6 +43,11 @@ namespace lab
         float*  coarse_inv32 = nullptr;
         int     coarse_n     = 0;
         int*    status       = nullptr; // device word counting waits that ran out (borrowed)
+        // this hierarchy's own count of them since it was last read, and its bound
+        // (polls; 0: kStreamWaitLimit) and held barrier (set only to test that path)
+        int*     timeouts   = nullptr;
+        unsigned wait_polls = 0;
+        int      wait_held  = 0;
         int     coarse_singular = 0;
     };
 

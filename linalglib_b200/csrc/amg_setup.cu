@@ -1239,6 +1239,8 @@ namespace lab
             cudaFree(h->coarse_inv);
         if(h->coarse_inv32)
             cudaFree(h->coarse_inv32);
+        if(h->timeouts)
+            cudaFree(h->timeouts);
         delete static_cast<lab_hier_s*>(h);
         return LAB_OK;
     }
@@ -1471,6 +1473,15 @@ LAB_API lab_status lab_amg_setup(lab_amg_kind kind, lab_csr A, int max_level, la
 LAB_API lab_status lab_hierarchy_destroy(lab_hierarchy h)
 {
     return hierarchy_release(h);
+}
+
+LAB_API lab_status lab_hierarchy_wait_control(lab_hierarchy h, int64_t polls, int held)
+{
+    LAB_ARG(h, "null hierarchy");
+    LAB_ARG(polls >= 0 && polls <= 0xffffffffll, "polls out of range");
+    h->wait_polls = (unsigned)polls;
+    h->wait_held  = held != 0;
+    return LAB_OK;
 }
 
 LAB_API lab_status lab_hierarchy_levels(lab_hierarchy h, int* n)

@@ -897,9 +897,27 @@ namespace lab
         }
         LAB_TRY(build_coarse(h, o->coarse, s));
         // the first call allocates, which a cycle inside a caller's capture must not
-        h->status   = device_status_word();
+        h->status = device_status_word();
+        if(!h->timeouts)
+        {
+            LAB_TRY(dalloc(&h->timeouts, 1, s));
+            LAB_CUDA(cudaMemsetAsync(h->timeouts, 0, sizeof(int), s));
+        }
         h->ws_ready = 1;
         return LAB_OK;
+    }
+
+    lab_status cycle_check(hierarchy_impl* h, cudaStream_t s)
+    {
+        if(!h->timeouts)
+            return LAB_OK;
+        int n = 0;
+        LAB_TRY(copy_d2h_sync(&n, h->timeouts, sizeof(n), s));
+        if(!n)
+            return LAB_OK;
+        LAB_CUDA(cudaMemsetAsync(h->timeouts, 0, sizeof(int), s));
+        set_error("AMG cycle: a wait for the operators of the last levels ran out");
+        return LAB_TIMEOUT;
     }
 
     // ================================================================ reductions

@@ -18,6 +18,10 @@ namespace lab
     // Synchronises; never called inside a graph capture.
     lab_status cycle_prepare(hierarchy_impl* h, const lab_amg_options* o, cudaStream_t s);
 
+    // Reads (and clears) the count of the cycles' waits that ran out: LAB_TIMEOUT if
+    // there was one (its cycle's result is NaN).  Synchronises.
+    lab_status cycle_check(hierarchy_impl* h, cudaStream_t s);
+
     // z = cycle(0; r) on level 0 (FP64 interface whatever the cycle precision).
     // With dot.out set, also (z, r) -> dot.out.  Enqueue only (capturable).
     lab_status cycle_precond(hierarchy_impl* h, const cyc_ctx& c, const double* r, double* z,

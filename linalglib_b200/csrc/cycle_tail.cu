@@ -88,8 +88,13 @@ namespace lab
         const double*  ainv; // coarsest n x n: dense inverse (o_v of its pass: local copy)
         int            nc;
         void*          dst; // the launch's result
+        int            ndst;
         const int*     skip;
-        int*           status; // counts waits that ran out
+        // counts of waits that ran out (the device's, the hierarchy's), the bound in
+        // polls, and 1 for an arrival that never comes (the test of the bound)
+        int *          status, *timeouts;
+        unsigned       polls;
+        int            held;
     };
 
     template <class T, class IT>
@@ -194,7 +199,7 @@ namespace lab
         }
         if(threadIdx.x == 0)
         {
-            mbar_init(&bar, 1);
+            mbar_init(&bar, 1 + a.held);
             fence_barrier_init();
             mbar_arrive_expect_tx(&bar, (unsigned)a.bytes);
         }
@@ -225,17 +230,23 @@ namespace lab
                 if(gc[u] >= 0)
                     xg[threadIdx.x + u * kTailNT] = g[u];
         }
-        // every copy has landed; a wait that runs out counts itself, drains (bounded)
-        // and leaves without writing the result
+        // every copy has landed; a wait that runs out makes the result NaN (no solve goes
+        // on with it), counts itself, drains (bounded) and leaves
         {
             bool ok = false;
-            for(unsigned i = 0; i < kStreamWaitLimit && !ok; i++)
+            for(unsigned i = 0; i < a.polls && !ok; i++)
                 ok = mbar_try_wait(&bar, 0);
             if(__syncthreads_or(!ok))
             {
+                if(!skip)
+                    for(int i = threadIdx.x; i < a.ndst; i += kTailNT)
+                        static_cast<T*>(a.dst)[i] = (T)__longlong_as_double(0x7ff8000000000000ll);
                 if(threadIdx.x == 0)
                 {
                     atomicAdd(a.status, 1);
+                    atomicAdd(a.timeouts, 1);
+                    if(a.held)
+                        mbar_arrive(&bar);
                     for(unsigned i = 0; i < kStreamWaitLimit && !mbar_try_wait(&bar, 0); i++)
                         ;
                 }
@@ -472,6 +483,7 @@ namespace lab
             }
             a.pass[a.npass - 1].out = 1;
             a.dst                   = dst;
+            a.ndst                  = a.pass[a.npass - 1].m;
             a.omega                 = o->omega;
         }
     };
@@ -535,8 +547,11 @@ namespace lab
     {
         tail_plan<T> t;
         t.build(h, c.o, l, edge, wr, cur, dst);
-        t.a.skip   = c.skip;
-        t.a.status = h->status;
+        t.a.skip     = c.skip;
+        t.a.status   = h->status;
+        t.a.timeouts = h->timeouts;
+        t.a.polls    = h->wait_polls ? h->wait_polls : kStreamWaitLimit;
+        t.a.held     = h->wait_held;
         static const cudaError_t attr = cudaFuncSetAttribute(
             k_tail<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem);
         LAB_CUDA(attr);

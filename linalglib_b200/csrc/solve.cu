@@ -1865,7 +1865,11 @@ LAB_API lab_status lab_amg_solve(lab_hierarchy h, const lab_amg_options* o, cons
     LAB_ARG(h && b && x && c, "null argument");
     LAB_TRY(check_options(o));
     LAB_TRY(ensure_init());
-    return amg_solve(h, o, b, x, c, info, to_stream(s));
+    const lab_status st = amg_solve(h, o, b, x, c, info, to_stream(s));
+    const lab_status e  = st == LAB_NAN ? cycle_check(h, to_stream(s)) : LAB_OK;
+    if(e != LAB_OK && info)
+        info->status = e;
+    return e != LAB_OK ? e : st;
 }
 
 LAB_API lab_status lab_precond_create_amg(lab_hierarchy h, const lab_amg_options* o,
@@ -1924,14 +1928,26 @@ LAB_API lab_status lab_precond_create_jacobi(lab_csr A, lab_precond* out, lab_st
     return LAB_OK;
 }
 
-// A triangular preconditioner's solves give up only if a row's dependencies never
-// arrive (a bug, not an input property): report it over the solver's status.
-static lab_status tri_status(lab_precond_s* M, lab_status st, cudaStream_t s)
+// A preconditioner's bounded waits run out only if what they wait for never arrives (a
+// bug, not an input property): report it over the solver's status.  A cycle's leaves NaN,
+// so its count is read only after a solve that ended with one.
+static lab_status wait_status(lab_precond M, lab_status st, lab_solve_info* info, lab_stream ls)
 {
-    lab_status e = tri_check(M->F, s);
-    if(e == LAB_OK && M->G)
-        e = tri_check(M->G, s);
-    return e != LAB_OK ? e : st;
+    cudaStream_t s = to_stream(ls);
+    lab_status   e = LAB_OK;
+    if(M && M->kind == 0 && st == LAB_NAN)
+        e = cycle_check(M->h, s);
+    if(M && M->kind >= 2 && st != LAB_BAD_ARG)
+    {
+        e = tri_check(M->F, s);
+        if(e == LAB_OK && M->G)
+            e = tri_check(M->G, s);
+    }
+    if(e == LAB_OK)
+        return st;
+    if(info)
+        info->status = e;
+    return e;
 }
 
 // ILU(0) / IC(0): factor a copy of A (ilu_precond::build, preconditioner.cpp:432-450;
@@ -2040,10 +2056,10 @@ LAB_API lab_status lab_pcg_solve(lab_csr A, lab_precond M, const double* b, doub
     LAB_TRY(ensure_init());
     if(!M)
         return cg_plain(A, b, x, c, info, to_stream(s));
-    if(M->kind == 0 && M->o.precision != LAB_PREC_FP64)
-        return pcg_refine(A, M, b, x, c, info, to_stream(s));
-    lab_status st = pcg_solve(A, M, b, x, c, info, to_stream(s));
-    return M->kind >= 2 && st != LAB_BAD_ARG ? tri_status(M, st, to_stream(s)) : st;
+    const lab_status st = M->kind == 0 && M->o.precision != LAB_PREC_FP64
+                              ? pcg_refine(A, M, b, x, c, info, to_stream(s))
+                              : pcg_solve(A, M, b, x, c, info, to_stream(s));
+    return wait_status(M, st, info, s);
 }
 
 LAB_API lab_status lab_pcg_solve_host(lab_csr A, lab_precond M, const double* bh, double* xh,
@@ -2061,8 +2077,7 @@ LAB_API lab_status lab_pcg_solve_host(lab_csr A, lab_precond M, const double* bh
                        : (M->kind == 0 && M->o.precision != LAB_PREC_FP64)
                              ? pcg_refine(A, M, b.get(), x.get(), c, info, s)
                              : pcg_solve(A, M, b.get(), x.get(), c, info, s);
-    if(M && M->kind >= 2 && st != LAB_BAD_ARG)
-        st = tri_status(M, st, s);
+    st = wait_status(M, st, info, ls);
     if(st != LAB_OK && st != LAB_NOT_CONVERGED && st != LAB_NAN)
         return st;
     LAB_CUDA(cudaMemcpyAsync(xh, x.get(), sizeof(double) * A->m, cudaMemcpyDeviceToHost, s));
@@ -2078,8 +2093,7 @@ LAB_API lab_status lab_gmres_solve(lab_csr A, lab_precond M, int restart, const 
     LAB_ARG(A->m == A->n, "GMRES needs a square matrix");
     LAB_ARG(restart >= 1, "restart must be >= 1");
     LAB_TRY(ensure_init());
-    lab_status st = gmres_solve(A, M, restart, b, x, c, info, to_stream(s));
-    return M && M->kind >= 2 && st != LAB_BAD_ARG ? tri_status(M, st, to_stream(s)) : st;
+    return wait_status(M, gmres_solve(A, M, restart, b, x, c, info, to_stream(s)), info, s);
 }
 
 __global__ void k_block_copy(const int32_t* __restrict__ rp, const int32_t* __restrict__ ci,
@@ -2163,7 +2177,8 @@ LAB_API lab_status lab_batched_pcg_solve(lab_csr A, lab_precond M, int nsys,
     seg_ops o;
     o.A = A;
     o.M = M;
-    return seg_solve(o, nsys, offsets, b, x, c, iterations, converged, info, s);
+    return wait_status(M, seg_solve(o, nsys, offsets, b, x, c, iterations, converged, info, s), info,
+                       ls);
 }
 
 LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, const double* B,
@@ -2214,7 +2229,8 @@ LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, c
     o.M     = M;
     o.multi = 1;
     o.n     = A->m;
-    return seg_solve(o, nrhs, off.data(), B, X, c, iterations, converged, info, s);
+    return wait_status(
+        M, seg_solve(o, nrhs, off.data(), B, X, c, iterations, converged, info, s), info, ls);
 }
 
 LAB_API lab_status lab_adjoint_solve(lab_csr A, lab_precond M, int symmetric, const double* g,
@@ -2229,11 +2245,11 @@ LAB_API lab_status lab_adjoint_solve(lab_csr A, lab_precond M, int symmetric, co
     {
         if(!M)
             return cg_plain(A, g, lambda, c, info, s);
-        return pcg_solve(A, M, g, lambda, c, info, s);
+        return wait_status(M, pcg_solve(A, M, g, lambda, c, info, s), info, ls);
     }
     lab_csr_impl* T = nullptr;
     LAB_TRY(transpose(A, &T, s));
-    lab_status st = gmres_solve(T, M, 50, g, lambda, c, info, s);
+    lab_status st = wait_status(M, gmres_solve(T, M, 50, g, lambda, c, info, s), info, ls);
     csr_release(T);
     return st;
 }

@@ -119,3 +119,43 @@ for precision in (L.PREC_FP64, L.PREC_FP32):
     p = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True,
                        timeout=300)
     assert p.returncode == 0, p.stderr[-2000:]
+
+
+def _timeouts(gpu):
+    import ctypes as C
+    n = C.c_int64()
+    L.call("lab_wait_timeouts", C.byref(n), gpu.stream_handle())
+    return n.value
+
+
+@pytest.mark.parametrize("precision", [L.PREC_FP64, L.PREC_FP32])
+@pytest.mark.parametrize("make", [lambda: P.poisson2d(61), lambda: P.poisson2d(100, 83)],
+                         ids=["with R and P", "without"])
+def test_tail_wait_that_runs_out(gpu, oracle, make, precision):
+    """The tail's wait for its operators is bounded.  Held back (a barrier that waits for
+    an arrival that never comes), the cycle's result is NaN, the wait is counted, every
+    solve returns LAB_TIMEOUT, and the next solves run as if nothing had been."""
+    A = make()
+    m = A[0].size - 1
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    H = gpu.Hierarchy(dA, kind=L.AMG_SA)
+    opts = gpu.amg_options(omega=2.0 / 3.0, precision=precision)
+    b = gpu.vec(np.random.default_rng(m).uniform(-1, 1, m))
+    M = gpu.Preconditioner.amg(H, opts)
+    want, info = gpu.pcg(dA, b, M=M)
+    L.call("lab_hierarchy_wait_control", H.h, 256, 1)
+    M = gpu.Preconditioner.amg(H, opts)
+    n0 = _timeouts(gpu)
+    assert np.isnan(M.apply(b).cpu().numpy()).all() and _timeouts(gpu) == n0 + 1
+    offsets = np.array([0, m], dtype=np.int64)
+    for solve in (lambda: gpu.pcg(dA, b, M=M), lambda: gpu.gmres(dA, b, M=M),
+                  lambda: gpu.adjoint_solve(dA, b, M), lambda: H.solve(b, options=opts),
+                  lambda: gpu.batched_pcg(dA, offsets, b, M)):
+        with pytest.raises(L.LabError) as e:
+            solve()
+        assert e.value.status == L.LAB_TIMEOUT
+    L.call("lab_hierarchy_wait_control", H.h, 0, 0)
+    M = gpu.Preconditioner.amg(H, opts)
+    n0 = _timeouts(gpu)
+    x, again = gpu.pcg(dA, b, M=M)
+    assert again.iterations == info.iterations and bool((x == want).all()) and _timeouts(gpu) == n0

@@ -602,9 +602,10 @@ namespace lab
     //
     // ctl[1] is the error flag, set when a warp waited idle_limit rounds without
     // progress; the other warps see it when they claim their next chunk or every
-    // 1024 idle rounds and return.  held (>= 0) is a row whose value is never
-    // written: the rows that depend on it can only run out of their wait (the test
-    // of this path).
+    // 1024 idle rounds.  From then on the rows that are not solved get kTriPending in x
+    // (a NaN, as nobody may go on with an earlier solve's values), and the launch ends
+    // with the last chunk.  held (>= 0) is a row whose value is never written: the rows
+    // that depend on it can only run out of their wait (the test of this path).
     template <bool LOWER, int PF>
     __global__ void __launch_bounds__(kTriBlock)
         k_trsv(const int32_t* __restrict__ ent_ptr, const int32_t* __restrict__ ent_col,
@@ -616,16 +617,28 @@ namespace lab
         if(skip && *skip)
             return;
         const int lane = threadIdx.x & 31;
+        if(held >= 0 && blockIdx.x == 0 && threadIdx.x == 0)
+            x[held] = __longlong_as_double((long long)kTriPending);
         for(;;)
         {
-            int base = 0;
+            int base = 0, given_up = 0;
             if(lane == 0)
-                base = ld_acquire(ctl + 1) ? m : atomicAdd(ctl, 32);
-            base = __shfl_sync(0xffffffffu, base, 0);
+            {
+                given_up = ld_acquire(ctl + 1);
+                base     = atomicAdd(ctl, 32);
+            }
+            base     = __shfl_sync(0xffffffffu, base, 0);
+            given_up = __shfl_sync(0xffffffffu, given_up, 0);
             if(base >= m)
                 return;
             const int t    = base + lane;
             bool      done = t >= m;
+            if(given_up)
+            {
+                if(!done)
+                    x[order[t]] = __longlong_as_double((long long)kTriPending);
+                continue;
+            }
             int       i = 0, k = 0, e = 0;
             double    acc = 0.0, d = 1.0, bi = 0.0;
             int       pc[PF];
@@ -724,14 +737,16 @@ namespace lab
                     idle = 0;
                 else
                 {
-                    if(++idle >= idle_limit)
+                    const bool out = ++idle >= idle_limit;
+                    if(out && lane == 0)
+                        atomicExch(ctl + 1, 1);
+                    if(out || ((idle & 1023u) == 0 &&
+                               __any_sync(0xffffffffu, ld_acquire(ctl + 1) != 0)))
                     {
-                        if(lane == 0)
-                            atomicExch(ctl + 1, 1);
-                        return;
+                        if(!done)
+                            x[i] = __longlong_as_double((long long)kTriPending);
+                        break;
                     }
-                    if((idle & 1023u) == 0 && __any_sync(0xffffffffu, ld_acquire(ctl + 1) != 0))
-                        return;
                     if(far)
                         __nanosleep(32);
                 }
@@ -952,6 +967,18 @@ namespace lab
             g    = gn;
             w += step;
         }
+        // given up: the rows of the warp's chunks from that one on whose value is pending get
+        // kTriPending in x, as on the grid (read back from where the values are; keeping
+        // track of them in the loop above cost 3 % of the 64^3 solve)
+        if(!ok)
+            for(w -= step; w < chunks; w += step)
+            {
+                const int i = get_head(w).x;
+                if(i >= 0 && xs[(w >> logc) * 32 + lane] == kTriPending)
+                    x[i] = __longlong_as_double((long long)kTriPending);
+            }
+        if(held >= 0 && rank == 0 && threadIdx.x == 0)
+            x[held] = __longlong_as_double((long long)kTriPending);
         __syncwarp();
         cluster_barrier(); // no CTA leaves while others may read its shared memory
     }

@@ -336,3 +336,35 @@ def test_trsv_bounded_wait_on_grid(gpu, oracle):
     L.call("lab_csrtrsv_wait_control", dA.h, 0, -1, gpu.stream_handle())
     x = dA.trsv(gpu.vec(b), lower=True)
     assert np.array_equal(_bits(x.cpu().numpy()), _bits(oracle.trsv(A, b, True, False)))
+
+
+@pytest.mark.parametrize("lower", [True, False])
+@pytest.mark.parametrize("make, held", [
+    (lambda: P.poisson3d(24), 5000),        # a row in the middle, 16 CTAs
+    (lambda: P.poisson2d(40), 800),         # one CTA
+    (lambda: _two_levels(9000), 4400),      # the grid
+], ids=["cluster", "one", "grid"])
+def test_trsv_rows_that_time_out_are_nan(gpu, oracle, make, held, lower):
+    """A solve that gives up leaves NaN in every row it did not solve (the held row's
+    dependents at least), and the solution in the others; an earlier solve's values
+    stay nowhere."""
+    from linalglib_b200 import _lib as L
+    A = make()[:3]
+    m = A[0].size - 1
+    b = np.random.default_rng(7).uniform(-1, 1, m)
+    want = oracle.trsv(A, b, lower, False)
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    row = held if lower else m - 1 - held
+    L.call("lab_csrtrsv_wait_control", dA.h, 1 << 12, row, gpu.stream_handle())
+    bx, x = gpu.vec(b), gpu.vec(np.full(m, 3.0))
+    st = L.lib().lab_csrtrsv(dA.h, int(lower), 0, gpu.ptr(bx), gpu.ptr(x), gpu.stream_handle())
+    assert st == L.LAB_TIMEOUT
+    x = x.cpu().numpy()
+    solved = ~np.isnan(x)
+    assert np.array_equal(_bits(x[solved]), _bits(want[solved]))
+    need = np.zeros(m, bool)  # the held row and the rows that depend on it
+    need[row] = True
+    for i in (range(row, m) if lower else range(row, -1, -1)):
+        c = A[1][A[0][i]:A[0][i + 1]]
+        need[i] |= bool(need[c[c < i] if lower else c[c > i]].any())
+    assert not solved[need].any()

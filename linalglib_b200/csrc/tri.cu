@@ -1048,15 +1048,27 @@ namespace lab
     //  - A mean level of 64 rows (two chunks) a CTA: fewer CTAs poll closer memory, more
     //    solve a level's chunks side by side (40^3, 542 rows a level: 16 CTAs 8.3 ms, 8
     //    8.6, 4 10.3; 100^2, 50 rows: 1 CTA 17.8 ms, 2 20.8), and as many as x needs.
-    //  - Up to 4096 rows a level: 16 SMs hold 4096 rows in flight, and a lower solve
-    //    with levels of 500 / 1500 / 3000 / 4096 / 4200 rows takes 277 / 165 / 116 / 90 us
-    //    here against 384 / 216 / 136 / 95 on the grid, which is level with it beyond.
-    static int tri_cluster(bool lower, const tri_sched& t, int m)
+    //  - 16 SMs hold 4096 rows in flight.  A level of up to that many takes 0.1 to 0.3 us
+    //    less here than on the grid (a lower solve with levels of 500 / 1500 / 3000 / 4096
+    //    rows: 277 / 165 / 116 / 90 us against 384 / 216 / 136 / 95), every 1000 rows a level
+    //    has beyond them about 0.2 us more.  So up to 1024 rows beyond 4096 for each level
+    //    without any: a level of 100,000 rows before 100 of 64 takes 111 us here and 136 on
+    //    the grid, 10 of 20,000 before 100 of 100 144 and 141, 20 of 10,000 before 60 of 100
+    //    120 and 112, 40 of 10,000 before 80 of 64 184 and 142.
+    constexpr int kTriClRows = 4096;
+    constexpr int kTriClMore = 1024;
+    static int    tri_cluster(bool lower, const tri_sched& t, int m)
     {
         const int levels = std::max(1, (int)t.ptr.size() - 1);
         const int chunks = (int)ceil_div(m, 32);
         const int width  = (int)ceil_div(m, levels);
-        if(width > 4096)
+        int64_t   beyond = 0;
+        for(size_t k = 0; k + 1 < t.ptr.size(); k++)
+        {
+            const int rows = t.ptr[k + 1] - t.ptr[k];
+            beyond += rows > kTriClRows ? rows - kTriClRows : -kTriClMore;
+        }
+        if(beyond > 0)
             return 0;
         int C = 1;
         while(C < kTriClMax && (C * 64 < width ||

@@ -368,3 +368,41 @@ def test_trsv_rows_that_time_out_are_nan(gpu, oracle, make, held, lower):
         c = A[1][A[0][i]:A[0][i + 1]]
         need[i] |= bool(need[c[c < i] if lower else c[c > i]].any())
     assert not solved[need].any()
+
+
+def _levels(widths):
+    """Lower triangle whose level k has widths[k] rows, each with one entry in level
+    k - 1 and the diagonal."""
+    rng = np.random.default_rng(len(widths))
+    rp, ci, v, base, below = [np.zeros(1, np.int64)], [], [], 0, None
+    for w in widths:
+        i = np.arange(base, base + w)
+        if below is None:
+            ci.append(i)
+        else:
+            ci.append(np.stack([below[0] + rng.integers(0, below[1], w), i], 1).reshape(-1))
+        v.append(np.where(ci[-1] >= base, 2.0, rng.uniform(-1, 1, ci[-1].size)))
+        rp.append(rp[-1][-1] + (ci[-1].size // w) * np.arange(1, w + 1))
+        below, base = (base, w), base + w
+    return tuple(np.concatenate(a).astype(t) for a, t in zip((rp, ci, v),
+                                                             (np.int32, np.int32, np.float64)))
+
+
+@pytest.mark.parametrize("widths, launches", [
+    ([20000] + [64] * 30, 1),          # one wide level and enough others: the cluster
+    ([20000] + [64] * 10, 2),          # too few others to make up for it: the grid
+    ([10000] * 40 + [64] * 80, 2),     # many wide levels, a mean of 3376 rows: the grid
+    ([4096] * 12, 1), ([4097] * 12, 2),
+], ids=["head", "short", "heads", "4096", "4097"])
+def test_trsv_form_by_level_widths(gpu, oracle, widths, launches):
+    """The form is chosen by the widths of the levels and not by their mean; the cluster
+    is one launch, the grid two."""
+    A = _levels(widths)
+    b = np.random.default_rng(8).uniform(-1, 1, A[0].size - 1)
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    x = dA.trsv(gpu.vec(b), lower=True)
+    assert np.array_equal(_bits(x.cpu().numpy()), _bits(oracle.trsv(A, b, True, False)))
+    bx = gpu.vec(b)
+    n0 = gpu.launch_count()
+    dA.trsv(bx, lower=True)
+    assert gpu.launch_count() - n0 == launches

@@ -45,3 +45,28 @@ def test_block_pcg(gpu, oracle, op, ncols, n1, n2):
     for k in range(ncols):
         r = B[k] - P.csr_matvec(*A, X[k])
         assert np.max(np.abs(r)) <= 2e-9 * max(np.max(np.abs(B[k] - P.csr_matvec(*A, X0[k]))), 1e-30)
+
+
+@pytest.mark.parametrize("ncols", [1, 2, 5, 33, 64])
+@pytest.mark.parametrize("n, nc", [(16, 64), (26, 170), (48, 545), (52, 647)])
+def test_block_dense_coarse_level(gpu, oracle, n, nc, ncols):
+    """A coarsest level solved by its dense inverse, on both sides of the number of rows
+    (four per SM) from which a CTA takes four of them, the last ones a remainder."""
+    A = P.poisson2d(n)
+    rng = np.random.default_rng(n + ncols)
+    B = np.stack([P.csr_matvec(*A, rng.uniform(-1, 1, n * n)) for _ in range(ncols)])
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    H = gpu.Hierarchy(dA, kind=L.AMG_SA, max_level=1)
+    assert H.A(1).m == nc
+    M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0))
+    X, iters, conv, info = gpu.multi_rhs_pcg(dA, gpu.vec(B).reshape(ncols, n * n), M,
+                                             control=gpu.iter_control(rel_tol=1e-9, abs_tol=0.0))
+    assert info.converged == 1 and np.all(conv == 1)
+    X = X.cpu().numpy()
+    Ho = oracle.amg_setup(A, kind=0, max_level=1)
+    for k in range(min(ncols, 3)):
+        xo, it, _ = Ho.pcg(B[k], omega=2.0 / 3.0, coarse=1, rel_tol=1e-9)
+        assert abs(int(iters[k]) - it) <= 1
+        assert np.max(np.abs(X[k] - xo)) <= 1e-5 * np.max(np.abs(xo))
+    for k in range(ncols):
+        assert np.max(np.abs(B[k] - P.csr_matvec(*A, X[k]))) <= 2e-9 * np.max(np.abs(B[k]))

@@ -2192,7 +2192,10 @@ LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, c
     LAB_TRY(spmv_analyse(A, s));
     if(M->kind == 0)
         LAB_TRY(cycle_prepare(M->h, &M->o, s));
-    if(M->kind == 0 && cycle_block_supported(M->h, &M->o) && M->h->A[0]->m == A->m)
+    // One column takes the single-vector cycle, whose last levels are one launch (8^3 1.08
+    // ms a solve, 64^3 3.36, in a block of two columns 1.36 and 3.76); two take 1.32 and
+    // 5.41 ms there, 1.34 and 3.75 in a block.
+    if(nrhs > 1 && M->kind == 0 && cycle_block_supported(M->h, &M->o) && M->h->A[0]->m == A->m)
     {
         // as few blocks as kBlkMax allows, of about equal size
         const int      nblk = (int)ceil_div<int64_t>(nrhs, kBlkMax);

@@ -70,3 +70,23 @@ def test_block_dense_coarse_level(gpu, oracle, n, nc, ncols):
         assert np.max(np.abs(X[k] - xo)) <= 1e-5 * np.max(np.abs(xo))
     for k in range(ncols):
         assert np.max(np.abs(B[k] - P.csr_matvec(*A, X[k]))) <= 2e-9 * np.max(np.abs(B[k]))
+
+
+@pytest.mark.parametrize("op", list(OPS))
+def test_one_column_takes_the_single_cycle(gpu, op):
+    """One right-hand side takes the single-vector cycle (whose last levels are one launch:
+    fewer launches than the block cycle of two columns makes in as many iterations)."""
+    A = OPS[op]()
+    m = A[0].size - 1
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    M = gpu.Preconditioner.amg(gpu.Hierarchy(dA, kind=L.AMG_SA), gpu.amg_options(omega=2.0 / 3.0))
+    b = gpu.vec(np.random.default_rng(m).uniform(-1, 1, m))
+    ctl = gpu.iter_control(rel_tol=1e-9, abs_tol=0.0)
+    launches, out = [], []
+    for k in (1, 2):
+        n0 = gpu.launch_count()
+        X, it, _, _ = gpu.multi_rhs_pcg(dA, b.expand(k, m).contiguous(), M, control=ctl)
+        launches.append((gpu.launch_count() - n0) / (int(it[0]) + 1))
+        out.append(X[0].cpu().numpy())
+    assert launches[0] < launches[1]
+    assert np.max(np.abs(out[0] - out[1])) <= 1e-5 * np.max(np.abs(out[0]))

@@ -2212,13 +2212,17 @@ LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, c
                           iterations ? iterations + k : nullptr, converged ? converged + k : nullptr,
                           &one, s);
             if(st != LAB_OK && st != LAB_NOT_CONVERGED && st != LAB_NAN)
+            {
+                cycle_release_block(M->h, true, s);
                 return st;
+            }
             if(st == LAB_NAN || worst == LAB_OK)
                 worst = st;
             all.iterations = std::max(all.iterations, one.iterations);
             all.converged &= one.converged;
             all.solve_ms += one.solve_ms;
         }
+        cycle_release_block(M->h, true, s);
         all.status = worst;
         if(info)
             *info = all;

@@ -90,3 +90,31 @@ def test_one_column_takes_the_single_cycle(gpu, op):
         out.append(X[0].cpu().numpy())
     assert launches[0] < launches[1]
     assert np.max(np.abs(out[0] - out[1])) <= 1e-5 * np.max(np.abs(out[0]))
+
+
+def test_block_scratch_is_given_back(gpu):
+    """The level scratch of a wide block does not stay allocated: after the solve the
+    pool holds no more than before it, but for a bounded rest."""
+    import ctypes as C
+    import torch
+    rt = C.CDLL("libcudart.so.12")
+    pool = C.c_void_p()
+    assert rt.cudaDeviceGetDefaultMemPool(C.byref(pool), 0) == 0
+
+    def used():
+        torch.cuda.synchronize()
+        v = C.c_uint64()
+        assert rt.cudaMemPoolGetAttribute(pool, 7, C.byref(v)) == 0  # UsedMemCurrent
+        return v.value
+
+    A = P.poisson3d(64)
+    m = A[0].size - 1
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    H = gpu.Hierarchy(dA, kind=L.AMG_SA)
+    M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0))
+    B = torch.rand((64, m), dtype=torch.float64, device="cuda")
+    gpu.multi_rhs_pcg(dA, B[:1], M)
+    before = used()
+    gpu.multi_rhs_pcg(dA, B, M)
+    rows = sum(H.A(l).m for l in range(H.levels + 1))
+    assert used() - before <= max(256 * rows, 64 << 20)

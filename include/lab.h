@@ -345,6 +345,10 @@ LAB_API lab_status lab_hierarchy_level(lab_hierarchy h, int level, lab_csr* A, l
                                        lab_csr* R);
 /* Setup timing of the last lab_amg_setup on this hierarchy, milliseconds. */
 LAB_API lab_status lab_hierarchy_setup_ms(lab_hierarchy h, double* ms);
+/* The most device memory, in bytes, that a block of right-hand sides may take for its
+ * vectors (lab_multi_rhs_pcg_solve with a preconditioner on h; 0, the default: what the
+ * device has).  Narrower blocks are used until two columns need more (LAB_OOM). */
+LAB_API lab_status lab_hierarchy_block_memory(lab_hierarchy h, int64_t bytes);
 /* The bound, in polls, of the waits in h's cycles (0: the default), and whether they wait
  * for something that never comes (to test the bound).  Set before solving with h:
  * iteration graphs captured earlier keep theirs. */
@@ -524,8 +528,11 @@ LAB_API lab_status lab_batched_pcg_solve(lab_csr A, lab_precond M, int nsys,
 LAB_API lab_status lab_batch_partition(int nsys, const int64_t* cost, int nparts, int* part);
 /* Block PCG for nrhs right-hand sides of one matrix: B and X are n x nrhs
  * column-major (leading dimension n).  Every column has its own scalars and
- * stopping test; the products with A use SpMM (one pass over A per block of 8
- * columns). */
+ * stopping test.  With an FP64 V-cycle of Jacobi sweeps up to 64 columns are solved
+ * together, each operator read once for all of them; that takes 56 n bytes of device
+ * memory a column and 32 bytes for each row of the coarser levels, and where they
+ * cannot be had narrower blocks are solved one after another.  A column's last bits
+ * depend on how many are solved with it (the order of its sums does). */
 LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, const double* B,
                                            double* X, const lab_iter_control* c, int* iterations,
                                            int* converged, lab_solve_info* info, lab_stream s);

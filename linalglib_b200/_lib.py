@@ -103,6 +103,7 @@ _SIGS = {
     "lab_hierarchy_destroy": [_p],
     "lab_hierarchy_levels": [_p, C.POINTER(_i)],
     "lab_hierarchy_level": [_p, _i, C.POINTER(_p), C.POINTER(_p), C.POINTER(_p)],
+    "lab_hierarchy_block_memory": [_p, _i64],
     "lab_hierarchy_wait_control": [_p, _i64, C.c_int],
     "lab_hierarchy_setup_ms": [_p, C.POINTER(_d)],
     "lab_csrtrsv": [_p, _i, _i, _p, _p, _p],

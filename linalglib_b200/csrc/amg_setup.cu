@@ -1475,6 +1475,14 @@ LAB_API lab_status lab_hierarchy_destroy(lab_hierarchy h)
     return hierarchy_release(h);
 }
 
+LAB_API lab_status lab_hierarchy_block_memory(lab_hierarchy h, int64_t bytes)
+{
+    LAB_ARG(h, "null hierarchy");
+    LAB_ARG(bytes >= 0, "negative size");
+    h->block_bytes = bytes;
+    return LAB_OK;
+}
+
 LAB_API lab_status lab_hierarchy_wait_control(lab_hierarchy h, int64_t polls, int held)
 {
     LAB_ARG(h, "null hierarchy");

@@ -83,11 +83,12 @@ namespace lab
                             double* r, cudaStream_t s);
     // Block V-cycle: whether the options are covered (V-cycle, Jacobi, FP64, 1x1 or
     // dense coarsest solve; call after cycle_prepare), the block workspace of at least ld
-    // columns (outside graph capture), its release, unless it is small when if_large is set,
-    // and z = cycle(0; r) on ld columns, with (z, r) per column into
+    // columns (outside graph capture; LAB_OOM also where it and vectors solve vectors of
+    // level 0 are more than the hierarchy's bound), its release, unless it is small when
+    // if_large is set, and z = cycle(0; r) on ld columns, with (z, r) per column into
     // dot.out when set.
     bool       cycle_block_supported(const hierarchy_impl* h, const lab_amg_options* o);
-    lab_status cycle_prepare_block(hierarchy_impl* h, int ld, cudaStream_t s);
+    lab_status cycle_prepare_block(hierarchy_impl* h, int ld, int vectors, cudaStream_t s);
     void       cycle_release_block(hierarchy_impl* h, bool if_large, cudaStream_t s);
     lab_status cycle_precond_block(hierarchy_impl* h, const cyc_ctx& c, int ld, const double* r,
                                    double* z, const blk_red& dot);

@@ -826,8 +826,17 @@ namespace lab
         return Ac->m <= 1 || (o->coarse == LAB_COARSE_DIRECT && h->coarse_inv);
     }
 
-    lab_status cycle_prepare_block(hierarchy_impl* h, int ld, cudaStream_t s)
+    lab_status cycle_prepare_block(hierarchy_impl* h, int ld, int vectors, cudaStream_t s)
     {
+        int64_t rows = (int64_t)(vectors + 2) * h->A[0]->m;
+        for(int l = 1; l <= h->levels; l++)
+            rows += 4 * h->A[l]->m;
+        const int64_t bytes = rows * ld * (int64_t)sizeof(double);
+        if(h->block_bytes && bytes > h->block_bytes)
+        {
+            set_error("a block of %d columns needs %lld bytes", ld, (long long)bytes);
+            return LAB_OOM;
+        }
         for(int l = 0; l <= h->levels; l++)
         {
             level_ws& w = h->ws[l];

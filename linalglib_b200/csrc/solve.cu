@@ -1685,7 +1685,7 @@ namespace lab
     {
         const int64_t n  = A->m;
         const int     ld = (ncols + 1) / 2 * 2;
-        LAB_TRY(cycle_prepare_block(M->h, ld, s));
+        LAB_TRY(cycle_prepare_block(M->h, ld, 5, s));
         dbuf<double>       x, r, z, p, q, sc, partial;
         dbuf<int>          sf, gflags;
         dbuf<unsigned int> counter;
@@ -2197,13 +2197,14 @@ LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, c
     // 5.41 ms there, 1.34 and 3.75 in a block.
     if(nrhs > 1 && M->kind == 0 && cycle_block_supported(M->h, &M->o) && M->h->A[0]->m == A->m)
     {
-        // as few blocks as kBlkMax allows, of about equal size
+        // as few blocks as kBlkMax allows, of about equal size; where memory does not last,
+        // half as wide (a block writes X at its end alone, so it can be solved again)
         const int      nblk = (int)ceil_div<int64_t>(nrhs, kBlkMax);
-        const int      per  = (int)ceil_div<int64_t>(nrhs, nblk);
+        int            per  = (int)ceil_div<int64_t>(nrhs, nblk);
         lab_solve_info all{};
         lab_status     worst = LAB_OK;
         all.converged        = 1;
-        for(int k = 0; k < nrhs; k += per)
+        for(int k = 0; k < nrhs;)
         {
             lab_solve_info   one{};
             const int        nc = std::min(per, nrhs - k);
@@ -2211,11 +2212,18 @@ LAB_API lab_status lab_multi_rhs_pcg_solve(lab_csr A, lab_precond M, int nrhs, c
                 blk_solve(A, M, nc, B + (int64_t)k * A->m, X + (int64_t)k * A->m, c,
                           iterations ? iterations + k : nullptr, converged ? converged + k : nullptr,
                           &one, s);
+            if(st == LAB_OOM && nc > 2)
+            {
+                cycle_release_block(M->h, false, s);
+                per = (nc + 1) / 2;
+                continue;
+            }
             if(st != LAB_OK && st != LAB_NOT_CONVERGED && st != LAB_NAN)
             {
                 cycle_release_block(M->h, true, s);
                 return st;
             }
+            k += nc;
             if(st == LAB_NAN || worst == LAB_OK)
                 worst = st;
             all.iterations = std::max(all.iterations, one.iterations);

@@ -92,6 +92,38 @@ def test_one_column_takes_the_single_cycle(gpu, op):
     assert np.max(np.abs(out[0] - out[1])) <= 1e-5 * np.max(np.abs(out[0]))
 
 
+@pytest.mark.parametrize("ncols", [64, 33])
+def test_block_width_by_memory(gpu, ncols):
+    """A block that does not fit the memory it may take is solved in narrower ones; two
+    columns that do not fit are an error that leaves X as it was.  Scratch of more than
+    64 MB is given back after the solve."""
+    A = P.poisson3d(40)
+    m = A[0].size - 1
+    rng = np.random.default_rng(ncols)
+    dA = gpu.CsrMatrix.from_arrays(*A)
+    H = gpu.Hierarchy(dA, kind=L.AMG_SA)
+    M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0))
+    B = gpu.vec(np.stack([P.csr_matvec(*A, rng.uniform(-1, 1, m)) for _ in range(ncols)]))
+    B = B.reshape(ncols, m)
+    ctl = gpu.iter_control(rel_tol=1e-9, abs_tol=0.0)
+    want, it0, conv, _ = gpu.multi_rhs_pcg(dA, B, M, control=ctl)
+    assert np.all(conv == 1)
+    want = want.cpu().numpy()
+    column = 8 * (7 * m + sum(4 * H.A(l).m for l in range(1, H.levels + 1)))
+    for width in (16, 3, 2):
+        L.call("lab_hierarchy_block_memory", H.h, column * (width + width % 2))
+        X, it, conv, info = gpu.multi_rhs_pcg(dA, B, M, control=ctl)
+        assert info.converged == 1 and np.all(conv == 1) and np.max(np.abs(it - it0)) <= 1
+        X = X.cpu().numpy()
+        assert np.max(np.abs(X - want)) <= 1e-5 * np.max(np.abs(want))
+    L.call("lab_hierarchy_block_memory", H.h, 2 * column - 1)
+    X = B.clone()
+    with pytest.raises(L.LabError) as e:
+        gpu.multi_rhs_pcg(dA, B, M, X=X, control=ctl)
+    assert e.value.status == L.LAB_OOM and bool((X == B).all())
+    L.call("lab_hierarchy_block_memory", H.h, 0)
+
+
 def test_block_scratch_is_given_back(gpu):
     """The level scratch of a wide block does not stay allocated: after the solve the
     pool holds no more than before it, but for a bounded rest."""

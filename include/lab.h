@@ -254,6 +254,9 @@ LAB_API lab_status lab_csr_scale_diagonal(lab_csr A, double scalar, lab_stream s
  * reference computes it).  Replaces csr_matrix::scale_by_inverse_diagonal
  * (csr_matrix.h:262; csr_matrix.cpp:277-299; host_scale.cpp:54-69). */
 LAB_API lab_status lab_csr_scale_by_inverse_diagonal(lab_csr A, lab_stream s);
+/* Dependency levels of a triangle and the form of its solves: by one cluster of so many
+ * CTAs, or (0) by the whole GPU.  Either output may be NULL. */
+LAB_API lab_status lab_csrtrsv_info(lab_csr A, int lower, int64_t* levels, int* ctas, lab_stream s);
 /* The bounded wait of the triangular solves on A (the lab_csrtrsv solves and the
  * ILU / IC / Gauss-Seidel / SOR / SSOR preconditioner applications).  A row waits
  * for its dependencies by polling; after idle_rounds rounds without progress
@@ -454,6 +457,14 @@ typedef struct lab_solve_info
     int    status;           /* lab_status of the solve */
 } lab_solve_info;
 
+/* The fused last levels of the V-cycles with options o on h, once a preconditioner with
+ * them exists: the level whose residual enters them (-1: none), and whether its
+ * restriction and prolongation are in the launch (at level 0 also only where its
+ * iterate starts and ends at a 16-byte boundary).  on = 0 gives every pass a launch of its
+ * own, with the same bits (graphs captured earlier keep theirs). */
+LAB_API lab_status lab_hierarchy_tail_info(lab_hierarchy h, const lab_amg_options* o, int* entry,
+                                           int* with_transfers);
+LAB_API lab_status lab_hierarchy_set_tail(lab_hierarchy h, int on);
 /* One cycle application x <- cycle(x; b) on level 0 (amg.cpp:144-513). */
 LAB_API lab_status lab_amg_cycle(lab_hierarchy h, const lab_amg_options* o, const double* b,
                                  double* x, lab_stream s);

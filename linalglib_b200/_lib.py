@@ -103,6 +103,8 @@ _SIGS = {
     "lab_hierarchy_destroy": [_p],
     "lab_hierarchy_levels": [_p, C.POINTER(_i)],
     "lab_hierarchy_level": [_p, _i, C.POINTER(_p), C.POINTER(_p), C.POINTER(_p)],
+    "lab_hierarchy_tail_info": [_p, _p, C.POINTER(_i), C.POINTER(_i)],
+    "lab_hierarchy_set_tail": [_p, _i],
     "lab_hierarchy_block_memory": [_p, _i64],
     "lab_hierarchy_wait_control": [_p, _i64, C.c_int],
     "lab_hierarchy_setup_ms": [_p, C.POINTER(_d)],
@@ -112,6 +114,7 @@ _SIGS = {
                      C.POINTER(_p), C.POINTER(_p)],
     "lab_mtx_write": [_p, _i64, _i64, _i64, _p, _p, _p],
     "lab_batch_partition": [_i, _p, _i, _p],
+    "lab_csrtrsv_info": [_p, _i, C.POINTER(_i64), C.POINTER(_i), _p],
     "lab_csrtrsv_wait_control": [_p, _i64, _i64, _p],
     "lab_csr_triangle": [_p, _i, C.POINTER(_p), _p],
     "lab_csr_scale_diagonal": [_p, _d, _p],

@@ -48,6 +48,7 @@ namespace lab
         int*     timeouts   = nullptr;
         unsigned wait_polls = 0;
         int      wait_held  = 0;
+        int      tail_off   = 0; // every pass of the last levels in its own launch
         int64_t  block_bytes = 0; // most that a block solve may allocate (0: no bound of its own)
         int     coarse_singular = 0;
     };

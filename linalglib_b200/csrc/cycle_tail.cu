@@ -506,7 +506,8 @@ namespace lab
     {
         const int L = h->levels, nl = L - l;
         if(o->cycle != LAB_CYCLE_V || o->smoother != LAB_SMOOTH_JACOBI || o->n1 < 1 ||
-           l >= L || nl > kTailMax || level_bf16(o, l) || !h->status)
+           l >= L || nl > kTailMax || level_bf16(o, l) || !h->status ||
+           h->tail_off)
             return TAIL_NONE;
         const int64_t nc = h->A[L]->m;
         if(nc != 1 && !(nc > 1 && nc <= kTailInv && o->coarse == LAB_COARSE_DIRECT && h->coarse_inv))

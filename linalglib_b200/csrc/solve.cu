@@ -1846,6 +1846,32 @@ static lab_status check_options(const lab_amg_options* o)
     return LAB_OK;
 }
 
+LAB_API lab_status lab_hierarchy_tail_info(lab_hierarchy h, const lab_amg_options* o, int* entry,
+                                           int* with_transfers)
+{
+    LAB_ARG(h && entry && with_transfers, "null argument");
+    LAB_TRY(check_options(o));
+    *entry          = -1;
+    *with_transfers = 0;
+    for(int l = 0; l < h->levels && *entry < 0; l++)
+    {
+        const int t = tail_ok(h, o, l);
+        if(t != TAIL_NONE)
+        {
+            *entry          = l;
+            *with_transfers = t == TAIL_EDGE;
+        }
+    }
+    return LAB_OK;
+}
+
+LAB_API lab_status lab_hierarchy_set_tail(lab_hierarchy h, int on)
+{
+    LAB_ARG(h, "null hierarchy");
+    h->tail_off = !on;
+    return LAB_OK;
+}
+
 LAB_API lab_status lab_amg_cycle(lab_hierarchy h, const lab_amg_options* o, const double* b,
                                  double* x, lab_stream ls)
 {

@@ -1549,6 +1549,21 @@ LAB_API lab_status lab_csrtrsv_wait_control(lab_csr A, int64_t idle_rounds, int6
     return LAB_OK;
 }
 
+LAB_API lab_status lab_csrtrsv_info(lab_csr A, int lower, int64_t* levels, int* ctas, lab_stream s)
+{
+    LAB_ARG(A, "null matrix");
+    LAB_ARG(A->m == A->n, "triangular analysis needs a square matrix");
+    LAB_TRY(ensure_init());
+    if(A->m > 0)
+        LAB_TRY(tri_analyse(A, to_stream(s)));
+    const tri_sched* t = A->m == 0 ? nullptr : lower ? &A->tri->lower : &A->tri->upper;
+    if(levels)
+        *levels = t ? (int64_t)t->ptr.size() - 1 : 0;
+    if(ctas)
+        *ctas = t ? t->cluster : 0;
+    return LAB_OK;
+}
+
 LAB_API lab_status lab_csr_triangle(lab_csr A, int upper, lab_csr* T, lab_stream s)
 {
     LAB_ARG(A && T, "null argument");

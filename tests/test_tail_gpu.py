@@ -1,6 +1,9 @@
-"""The fused V-cycle tail (csrc/cycle_tail.cu) against the oracle's V-cycle: entry at
-level 0 (few rows; odd and even sizes, an odd address), with and without the entry
-level's restriction and prolongation in the launch, several sweeps, FP64 and FP32."""
+"""The fused V-cycle tail (csrc/cycle_tail.cu) against the oracle's V-cycle and, bit for
+bit, against the cycle with every pass in its own launch: entry at level 0 (few rows; odd
+and even sizes, an odd address), with and without the entry level's restriction and
+prolongation in the launch, several sweeps, FP64 and FP32."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -9,19 +12,27 @@ from linalglib_b200 import problems as P
 
 pytestmark = pytest.mark.gpu
 
-CASES = [
-    ("2d 11", lambda: P.poisson2d(11)),           # entry 0, odd number of rows
-    ("2d 12", lambda: P.poisson2d(12)),           # entry 0
-    ("2d 61", lambda: P.poisson2d(61)),           # entry 1 with R and P
-    ("2d 100x83", lambda: P.poisson2d(100, 83)),  # entry 1 without R and P
-    ("3d 13", lambda: P.poisson3d(13)),           # long rows
-    ("27pt 12", lambda: P.diffusion27(12)),
+CASES = [  # with the entry level and whether R and P are in the launch
+    ("2d 11", lambda: P.poisson2d(11), 0, 1),  # odd: in the launch for no FP64 iterate
+    ("2d 12", lambda: P.poisson2d(12), 0, 1),
+    ("2d 40", lambda: P.poisson2d(40), 0, 0),
+    ("2d 61", lambda: P.poisson2d(61), 1, 1),
+    ("2d 100x83", lambda: P.poisson2d(100, 83), 1, 0),
+    ("3d 13", lambda: P.poisson3d(13), 1, 1),  # long rows
+    ("3d 24", lambda: P.poisson3d(24), 2, 1),
+    ("27pt 12", lambda: P.diffusion27(12), 1, 1),
 ]
 
 
+def _tail_info(H, opts):
+    entry, transfers = C.c_int(), C.c_int()
+    L.call("lab_hierarchy_tail_info", H.h, C.byref(opts), C.byref(entry), C.byref(transfers))
+    return entry.value, transfers.value
+
+
 @pytest.mark.parametrize("n1, n2", [(1, 1), (2, 1), (1, 0), (3, 2)])
-@pytest.mark.parametrize("name, make", CASES, ids=[c[0] for c in CASES])
-def test_tail_matches_oracle_cycle(gpu, oracle, name, make, n1, n2):
+@pytest.mark.parametrize("name, make, entry, transfers", CASES, ids=[c[0] for c in CASES])
+def test_tail_matches_oracle_cycle(gpu, oracle, name, make, entry, transfers, n1, n2):
     import torch
     A = make()
     m = A[0].size - 1
@@ -31,13 +42,19 @@ def test_tail_matches_oracle_cycle(gpu, oracle, name, make, n1, n2):
     # sums of at most ~200 products on each of a few dozen passes: 2^-53 and 2^-24 times
     # a few hundred, in the norm of the result
     for precision, tol in ((L.PREC_FP64, 1e-12), (L.PREC_FP32, 4e-5)):
-        M = gpu.Preconditioner.amg(H, gpu.amg_options(n1=n1, n2=n2, omega=2.0 / 3.0,
-                                                      precision=precision))
+        opts = gpu.amg_options(n1=n1, n2=n2, omega=2.0 / 3.0, precision=precision)
+        M = gpu.Preconditioner.amg(H, opts)
+        L.call("lab_hierarchy_set_tail", H.h, 0)
+        assert _tail_info(H, opts) == (-1, 0)
+        passes = M.apply(gpu.vec(r)).cpu().numpy()
+        L.call("lab_hierarchy_set_tail", H.h, 1)
+        assert _tail_info(H, opts) == (entry, transfers)
         for shift in (0, 1):  # z at a 16-byte boundary and 8 bytes off it
             z = torch.full((m + 3,), 7.0, dtype=torch.float64, device="cuda")
             M.apply(gpu.vec(r), z[shift:shift + m])
             z = z.cpu().numpy()
             assert np.max(np.abs(z[shift:shift + m] - zo)) <= tol * np.max(np.abs(zo))
+            assert np.array_equal(z[shift:shift + m].view(np.int64), passes.view(np.int64))
             assert np.all(z[:shift] == 7.0) and np.all(z[shift + m:] == 7.0)
 
 
@@ -74,6 +91,10 @@ def test_tail_empty_rows(gpu, oracle, make, lanes):
         M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0, precision=precision))
         z = M.apply(gpu.vec(r)).cpu().numpy()
         assert np.max(np.abs(z - zo)) <= tol * np.max(np.abs(zo))
+        L.call("lab_hierarchy_set_tail", H.h, 0)
+        passes = M.apply(gpu.vec(r)).cpu().numpy()
+        L.call("lab_hierarchy_set_tail", H.h, 1)
+        assert np.array_equal(z.view(np.int64), passes.view(np.int64))
 
 
 @pytest.mark.parametrize("n, launches", [(14, 3), (16, 3), (18, 5), (20, 5), (26, 5)])
@@ -122,7 +143,6 @@ for precision in (L.PREC_FP64, L.PREC_FP32):
 
 
 def _timeouts(gpu):
-    import ctypes as C
     n = C.c_int64()
     L.call("lab_wait_timeouts", C.byref(n), gpu.stream_handle())
     return n.value

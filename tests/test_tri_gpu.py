@@ -304,20 +304,30 @@ def _two_levels(n):
     return rp.astype(np.int32), ci.reshape(-1).astype(np.int32), v.reshape(-1)
 
 
-@pytest.mark.parametrize("make", [
-    lambda: P.poisson2d(130),       # levels of 65 rows: clusters of 2 CTAs
-    lambda: P.poisson3d(20),        # 138: 4
-    lambda: P.poisson3d(30),        # 307: 8
-    lambda: P.poisson3d(41),        # 570: 16
-    lambda: P.poisson2d(700),       # more than 16 CTAs' shared memory holds: the grid
-    lambda: _two_levels(9000),      # wide and shallow: the grid
-], ids=["c2", "c4", "c8", "c16", "large", "wide"])
-def test_trsv_cluster_sizes_bit_exact(gpu, oracle, make):
+def _ctas(gpu, dA, lower):
+    import ctypes as C
+    from linalglib_b200 import _lib as L
+    n, c = C.c_int64(), C.c_int()
+    L.call("lab_csrtrsv_info", dA.h, int(lower), C.byref(n), C.byref(c), gpu.stream_handle())
+    return c.value
+
+
+@pytest.mark.parametrize("make, ctas", [
+    (lambda: P.poisson2d(40), 1),
+    (lambda: P.poisson2d(130), 2),       # levels of 65 rows
+    (lambda: P.poisson3d(20), 4),        # 138
+    (lambda: P.poisson3d(30), 8),        # 307
+    (lambda: P.poisson3d(41), 16),       # 570
+    (lambda: P.poisson2d(700), 0),       # more than 16 CTAs' shared memory holds: the grid
+    (lambda: _two_levels(9000), 0),      # wide and shallow: the grid
+], ids=["c1", "c2", "c4", "c8", "c16", "large", "wide"])
+def test_trsv_cluster_sizes_bit_exact(gpu, oracle, make, ctas):
     A = make()[:3]
     b = np.random.default_rng(5).uniform(-1, 1, A[0].size - 1)
     dA = gpu.CsrMatrix.from_arrays(*A)
     for lower in (True, False):
         want = _bits(oracle.trsv(A, b, lower, False))
+        assert _ctas(gpu, dA, lower) == ctas
         for _ in range(2):
             x = dA.trsv(gpu.vec(b), lower=lower, unit_diag=False)
             assert np.array_equal(_bits(x.cpu().numpy()), want)
@@ -340,7 +350,7 @@ def test_trsv_bounded_wait_on_grid(gpu, oracle):
 
 @pytest.mark.parametrize("lower", [True, False])
 @pytest.mark.parametrize("make, held", [
-    (lambda: P.poisson3d(24), 5000),        # a row in the middle, 16 CTAs
+    (lambda: P.poisson3d(24), 5000),        # a row in the middle, 4 CTAs
     (lambda: P.poisson2d(40), 800),         # one CTA
     (lambda: _two_levels(9000), 4400),      # the grid
 ], ids=["cluster", "one", "grid"])
@@ -405,4 +415,4 @@ def test_trsv_form_by_level_widths(gpu, oracle, widths, launches):
     bx = gpu.vec(b)
     n0 = gpu.launch_count()
     dA.trsv(bx, lower=True)
-    assert gpu.launch_count() - n0 == launches
+    assert gpu.launch_count() - n0 == launches and (_ctas(gpu, dA, True) > 0) == (launches == 1)

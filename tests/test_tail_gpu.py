@@ -88,7 +88,9 @@ def test_tail_empty_rows(gpu, oracle, make, lanes):
             for M in (H.P(l), H.R(l)):
                 M.set_algorithm(L.SPMV_VECTOR, lanes)
     for precision, tol in ((L.PREC_FP64, 1e-12), (L.PREC_FP32, 4e-5)):
-        M = gpu.Preconditioner.amg(H, gpu.amg_options(omega=2.0 / 3.0, precision=precision))
+        opts = gpu.amg_options(omega=2.0 / 3.0, precision=precision)
+        M = gpu.Preconditioner.amg(H, opts)
+        assert _tail_info(H, opts)[0] == (1 if m > 1000 else 0)
         z = M.apply(gpu.vec(r)).cpu().numpy()
         assert np.max(np.abs(z - zo)) <= tol * np.max(np.abs(zo))
         L.call("lab_hierarchy_set_tail", H.h, 0)
@@ -179,3 +181,26 @@ def test_tail_wait_that_runs_out(gpu, oracle, make, precision):
     n0 = _timeouts(gpu)
     x, again = gpu.pcg(dA, b, M=M)
     assert again.iterations == info.iterations and bool((x == want).all()) and _timeouts(gpu) == n0
+
+
+@pytest.mark.parametrize("alg, lanes", [(L.SPMV_ROWSEQ, 0), (L.SPMV_VECTOR, 4),
+                                        (L.SPMV_VECTOR_STREAM, 8), (L.SPMV_VECTOR_HALO, 4),
+                                        (L.SPMV_VECTOR_HALO, 32)])
+def test_tail_keeps_the_order_of_the_schedules(gpu, alg, lanes):
+    """The tail sums a row in the order of its operator's schedule, also where that is
+    the streamed or the halo form of several lanes a row."""
+    A = P.poisson2d(61)
+    H = gpu.Hierarchy(gpu.CsrMatrix.from_arrays(*A), kind=L.AMG_SA)
+    for l in range(1, H.levels):
+        for M in (H.A(l), H.P(l), H.R(l)):
+            M.set_algorithm(alg, lanes)
+    r = gpu.vec(np.random.default_rng(61).uniform(-1, 1, 61 * 61))
+    for precision in (L.PREC_FP64, L.PREC_FP32):
+        opts = gpu.amg_options(n1=2, n2=2, omega=2.0 / 3.0, precision=precision)
+        M = gpu.Preconditioner.amg(H, opts)
+        assert _tail_info(H, opts)[0] == 1
+        z = M.apply(r)
+        L.call("lab_hierarchy_set_tail", H.h, 0)
+        passes = M.apply(r)
+        L.call("lab_hierarchy_set_tail", H.h, 1)
+        assert bool((z == passes).all())

@@ -443,9 +443,18 @@ namespace lab
         int      claims;
     };
 
-    __device__ __forceinline__ unsigned hash_slot(int c, unsigned mask)
+    // Multiplicative hashing by 2^32 / the golden ratio, high bits (Knuth, The Art of
+    // Computer Programming 3, section 6.4): runs of consecutive columns, which a
+    // product's rows are made of, land evenly spread.  (Bits 7 and up of the product
+    // put every fifth column next to the first: rows of A_1 P_1 of a 7-point operator
+    // took 6.1 probes for the slowest lane of a warp, now 3.7.  SA setup, 80^3 weighted
+    // graph Laplacian 9.17 -> 8.77 ms, 27-point 64^3 10.33 -> 10.18 ms, 7-point 128^3
+    // unchanged.  A plain read of the slot before the compare-and-swap changed nothing.)
+    template <int HS>
+    __device__ __forceinline__ unsigned hash_slot(int c)
     {
-        return ((unsigned)c * 2654435761u >> 7) & mask;
+        static_assert(HS >= 2 && (HS & (HS - 1)) == 0, "a power of two");
+        return (unsigned)c * 2654435769u >> (__builtin_clz((unsigned)HS) + 1);
     }
 
     __device__ __forceinline__ int warp_inclusive_sum(int v)
@@ -466,7 +475,7 @@ namespace lab
     __device__ __forceinline__ unsigned hash_claim(int* key, int col, bool* isnew)
     {
         constexpr unsigned mask = HS - 1;
-        unsigned           slot = hash_slot(col, mask);
+        unsigned           slot = hash_slot<HS>(col);
         *isnew                  = false;
         for(unsigned probe = 0; probe < HS; probe++)
         {

@@ -447,9 +447,11 @@ namespace lab
     // Computer Programming 3, section 6.4): runs of consecutive columns, which a
     // product's rows are made of, land evenly spread.  (Bits 7 and up of the product
     // put every fifth column next to the first: rows of A_1 P_1 of a 7-point operator
-    // took 6.1 probes for the slowest lane of a warp, now 3.7.  SA setup, 80^3 weighted
-    // graph Laplacian 9.17 -> 8.77 ms, 27-point 64^3 10.33 -> 10.18 ms, 7-point 128^3
-    // unchanged.  A plain read of the slot before the compare-and-swap changed nothing.)
+    // took 6.1 probes for the slowest lane of a warp, now 3.7.  Worth about 1 % of an SA
+    // setup, both forms in turn on one GPU: weighted graph Laplacian 80^3 8.85 -> 8.71 ms
+    // and 100^3 12.25 -> 12.36, 27-point 64^3 with the first application 10.31 -> 10.21,
+    // 7-point 64^3 6.74 -> 6.69, 128^3 20.0 with both.  A plain read of the slot before the
+    // compare-and-swap changed nothing.)
     template <int HS>
     __device__ __forceinline__ unsigned hash_slot(int c)
     {

@@ -261,9 +261,10 @@ LAB_API lab_status lab_csrtrsv_info(lab_csr A, int lower, int64_t* levels, int* 
  * ILU / IC / Gauss-Seidel / SOR / SSOR preconditioner applications).  A row waits
  * for its dependencies by polling; after idle_rounds rounds without progress
  * (0: the default, 2^26) its warp gives up, the launch returns and the call
- * reports LAB_TIMEOUT instead of hanging, with NaN in the rows not solved.  held_row >= 0 names a row whose value
- * the solves never write, so the rows that depend on it run out of their wait:
- * a test of that path (-1: none, the normal setting).  No reference counterpart
+ * reports LAB_TIMEOUT instead of hanging, with NaN in the rows not solved.
+ * held_row >= 0 names a row whose value the solves never write, so the rows that
+ * depend on it run out of their wait: a test of that path (-1: none, the normal
+ * setting).  No reference counterpart
  * (the reference's host solves are sequential loops, host_csrtrsv.cpp:36-90). */
 LAB_API lab_status lab_csrtrsv_wait_control(lab_csr A, int64_t idle_rounds, int64_t held_row,
                                             lab_stream s);
